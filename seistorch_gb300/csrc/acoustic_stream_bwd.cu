@@ -125,15 +125,10 @@ __global__ void __launch_bounds__(32 * NWP, TZ / NWP <= 2 ? (PTM >= 2 ? 3 : 4) :
     // adjoint sources (R^T of the record gather) into the injection tile;
     // every warp zeroes its own rows of it after reading them
     if (has_rec) {
-      const int* rp = a.rec_row_ptr + (long long)g.b * a.nz;
-      for (int lr = wid; lr < TZ && g.z0 + lr < a.nz; lr += NWP) {
-        const int z = g.z0 + lr;
-        const int p1 = rp[z + 1];
-        for (int q = rp[z] + lane; q < p1; q += 32) {
-          const int rx = a.rec_x[q] - g.x0;
-          if (rx >= 0 && rx < TX) atomicAdd(sinj + lr * TX + rx, a.resid[(long long)a.rec_col[q] * a.nch]);
-        }
-      }
+      tile_receivers<TZ, NWP>(a.rec_row_ptr + (long long)g.b * a.nz, a.rec_x, a.rec_col, lane, wid, g.x0, g.z0, a.nz,
+                              [&](int lr, int rx, int col) {
+                                atomicAdd(sinj + lr * TX + rx, __ldg(a.resid + (long long)col * a.nch));
+                              });
       __syncthreads();
     }
     if (!mbar_wait(&bars[stage], (k / S) & 1, a.status)) s_abort = 1;

@@ -121,6 +121,41 @@ __device__ __forceinline__ void apply_sources(const WarpSrc& s, int i, int lane,
   }
 }
 
+// The receivers of shot b in the rows [z0, z0 + TZ) and columns [x0, x0 + TX)
+// of a tile: f(row in tile, column in tile, rec_col) for each.  The rows of a
+// shot are adjacent in the table, so all NWP warps of the CTA walk the band's
+// receivers as one range, eight column loads per lane in flight (the columns
+// of a row need not be sorted); the row of a receiver comes from the band's
+// row pointers, one per lane.  With the receivers of a row walked by one warp
+// and one load in flight, a tile on a row of 1000 receivers took about 10 us.
+template <int TZ, int NWP, class F>
+__device__ __forceinline__ void tile_receivers(const int* rp, const int* rec_x, const int* rec_col, int lane, int wid,
+                                               int x0, int z0, int nz, const F& f) {
+  static_assert(TZ <= 32, "one row pointer per lane");
+  constexpr int U = 8;
+  const int rows = min(TZ, nz - z0);
+  const int pv = __ldg(rp + z0 + min(lane, rows - 1));  // first receiver of row `lane`
+  const int p1 = __ldg(rp + z0 + rows);
+  const int p0 = __shfl_sync(FULL, pv, 0);
+  for (int q0 = p0 + wid * 32; q0 < p1; q0 += 32 * NWP * U) {
+    int rx[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int q = q0 + u * 32 * NWP + lane;
+      rx[u] = q < p1 ? __ldg(rec_x + q) - x0 : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int q = q0 + u * 32 * NWP + lane;
+      const bool in = rx[u] >= 0 && rx[u] < TX;
+      if (!__any_sync(FULL, in)) continue;
+      int lr = 0;  // the last row whose first receiver is at or before q
+      for (int r = 1; r < rows; ++r) lr += __shfl_sync(FULL, pv, r) <= q ? 1 : 0;
+      if (in) f(lr, rx[u], __ldg(rec_col + q));
+    }
+  }
+}
+
 // This CTA's share of a boundary-ring copy between a field
 // [nshots][nz][pitch] and its slots [nshots][ring.size] (slot order of
 // Ring::index): scatter = slots -> field, else field -> slots.  Four
