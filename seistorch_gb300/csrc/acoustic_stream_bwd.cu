@@ -74,14 +74,17 @@ __global__ void __launch_bounds__(32 * NWP, TZ / NWP <= 2 ? (PTM >= 2 ? 3 : 4) :
     for (int s = 0; s < S; ++s) mbar_init(&bars[s], 1);
     fence_mbar_init();
     s_abort = 0;
+  }
+  for (int i = tid; i < Lay::PF / 4; i += 32 * NWP) sts4(sinj + 4 * i, make_float4(0.f, 0.f, 0.f, 0.f));
+  pdl_wait();
+  pdl_trigger();
+  if (tid == 0)
     for (int s = 0; s < S; ++s)
       if ((int)blockIdx.x + s * G < ntiles) issue(blockIdx.x + s * G, s);
-  }
   // the saved ring of U_{j-2}, each CTA a share while its first boxes load:
   // the tiles never write ring cells, and nothing in this launch reads U_{j-2}
   if (a.do_recon && a.ring_in != nullptr)
     ring_copy_share(a.ring, a.nshots, a.pitch, a.sstride, a.uout, const_cast<float*>(a.ring_in), true);
-  for (int i = tid; i < Lay::PF / 4; i += 32 * NWP) sts4(sinj + 4 * i, make_float4(0.f, 0.f, 0.f, 0.f));
   __syncthreads();
   int k = 0;
   for (int t = blockIdx.x; t < ntiles; t += G, ++k) {
@@ -100,8 +103,8 @@ __global__ void __launch_bounds__(32 * NWP, TZ / NWP <= 2 ? (PTM >= 2 ? 3 : 4) :
       if (xin && z < a.nz) {
         const long long mo = (long long)z * a.pitch + x;
         if constexpr (PTM == 0) {
-          vun[i] = ldg4(a.unext + fbase + mo);
-          vn2[i] = ldg4(a.n2 + fbase + mo);
+          vun[i] = ldf4(a.unext + fbase + mo);
+          vn2[i] = ldf4(a.n2 + fbase + mo);
         }
         if constexpr (PTM <= 1) {
           vg[i] = ldg4(a.g + mo);
@@ -239,9 +242,8 @@ static cudaError_t bwd_tile_t(const CUtensorMap* maps, const AcBwdStreamArgs& a,
     blocks = resident_blocks(kern, 32 * NWP, smem);
   }
   const int tiles = a.nshots * a.ntx * a.nzc;
-  kern<<<(unsigned)(tiles < blocks ? tiles : blocks), 32 * NWP, smem, s>>>(maps[0], maps[1], maps[2], maps[3],
-                                                                             maps[4], a);
-  return cudaGetLastError();
+  return launch_pdl(kern, dim3((unsigned)(tiles < blocks ? tiles : blocks)), dim3(32 * NWP), smem, s, maps[0], maps[1],
+                    maps[2], maps[3], maps[4], a);
 }
 
 template <int R>

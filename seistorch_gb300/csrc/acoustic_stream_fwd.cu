@@ -20,9 +20,9 @@ struct StageField {
   __device__ __forceinline__ float U(int z, int x) const {
     const int r = z - zt, c = x - xt;
     if (r >= 0 && r < rows && c >= 0 && c < w) return su[r * w + c];
-    return __ldg(u + base + (long long)z * pitch + x);
+    return ldf(u + base + (long long)z * pitch + x);
   }
-  __device__ __forceinline__ float P(int z, int x) const { return __ldg(um + base + (long long)z * pitch + x); }
+  __device__ __forceinline__ float P(int z, int x) const { return ldf(um + base + (long long)z * pitch + x); }
 };
 
 // The one-way blend of four cells of a row that all take the same single
@@ -183,9 +183,12 @@ __device__ __forceinline__ void fwd_tiles(const P& prov, const Pre& pre = Pre{})
     for (int s = 0; s < S; ++s) mbar_init(&bars[s], 1);
     fence_mbar_init();
     s_abort = 0;
+  }
+  pdl_wait();
+  pdl_trigger();
+  if (tid == 0)
     for (int s = 0; s < S; ++s)
       if ((int)blockIdx.x + s * G < ntiles) issue(blockIdx.x + s * G, s);
-  }
   pre();
   __syncthreads();
   int k = 0;
@@ -213,12 +216,12 @@ __device__ __forceinline__ void fwd_tiles(const P& prov, const Pre& pre = Pre{})
       const int z = zw + i;
       if (xin && z < a.nz) {
         const long long mo = (long long)z * a.pitch + x;
-        if (!PT) vm[i] = ldg4(a.um + (long long)b0 * a.sstride + mo);
+        if (!PT) vm[i] = ldf4(a.um + (long long)b0 * a.sstride + mo);
         vg[i] = ldg4(a.g + mo);
         vk[i] = ldg4(a.k + mo);
         if constexpr (HB == 2) vkz[i] = ldg4(a.kz + mo);
         if constexpr (HB == 1) vbn[i] = (bnp != nullptr && (a.born_in != nullptr || a.born_out != nullptr))
-                                            ? ldg4(bnp + mo) : make_float4(0.f, 0.f, 0.f, 0.f);
+                                            ? ldf4(bnp + mo) : make_float4(0.f, 0.f, 0.f, 0.f);
         if constexpr (HB == 3) {
 #pragma unroll
           for (int q = 0; q < 5; ++q) vrc[i][q] = ldg4(a.rho_c + q * (long long)a.nz * a.pitch + mo);
@@ -337,21 +340,21 @@ __device__ __forceinline__ void fwd_tiles(const P& prov, const Pre& pre = Pre{})
               auto urow = [&](int zz) -> float4 {
                 const int r = zz - (g.z0 - R);
                 return (r >= 0 && r < TZ + 2 * R) ? lds4(su + r * UW + LO + 4 * lane)
-                                                  : ldg4(a.u + fbase + (long long)zz * a.pitch + x);
+                                                  : ldf4(a.u + fbase + (long long)zz * a.pitch + x);
               };
               U1 = urow(z + dz);
               U2 = urow(z + 2 * dz);
-              P1 = ldg4(a.um + fbase + ro + dz * (long long)a.pitch);
+              P1 = ldf4(a.um + fbase + ro + dz * (long long)a.pitch);
             } else if (side == 2) {
               const float4 r4 = lds4(srow + LO + 4 + 4 * lane);
               U1 = make_float4(c.y, c.z, c.w, r4.x);
               U2 = make_float4(c.z, c.w, r4.x, r4.y);
-              P1 = make_float4(vm[i].y, vm[i].z, vm[i].w, __ldg(a.um + fbase + ro + 4));
+              P1 = make_float4(vm[i].y, vm[i].z, vm[i].w, ldf(a.um + fbase + ro + 4));
             } else {
               const float4 l4 = lds4(srow + LO - 4 + 4 * lane);
               U1 = make_float4(l4.w, c.x, c.y, c.z);
               U2 = make_float4(l4.z, l4.w, c.x, c.y);
-              P1 = make_float4(__ldg(a.um + fbase + ro - 1), vm[i].x, vm[i].y, vm[i].z);
+              P1 = make_float4(ldf(a.um + fbase + ro - 1), vm[i].x, vm[i].y, vm[i].z);
             }
             y = blend4(y, c, U1, U2, vm[i], P1, cv, bv, a.lamf, a.muf);
           } else {
@@ -449,7 +452,8 @@ static cudaError_t fwd_tile_t(const AcFwdBatch<MAXG>& b, cudaStream_t s, bool pr
     const AcStreamArgs& a = b.g[0];
     const int tiles = (a.nshots + SB - 1) / SB * a.ntx * a.nzc;
     if (tiles <= 0) return cudaSuccess;
-    kern<<<(unsigned)(tiles < blocks ? tiles : blocks), 32 * NWP, smem, s>>>(b.tm_u[0], b.tm_um[0], b.g[0]);
+    return launch_pdl(kern, dim3((unsigned)(tiles < blocks ? tiles : blocks)), dim3(32 * NWP), smem, s, b.tm_u[0],
+                      b.tm_um[0], b.g[0]);
   } else {
     auto kern = acoustic_fwd_batch_kernel<R, TZ, NWP, S, PT, MAXG>;
     if (blocks == 0) {
@@ -460,9 +464,8 @@ static cudaError_t fwd_tile_t(const AcFwdBatch<MAXG>& b, cudaStream_t s, bool pr
     if (prepare_only) return cudaSuccess;
     const int tiles = b.tile0[b.ngroups];
     if (tiles <= 0) return cudaSuccess;
-    kern<<<(unsigned)(tiles < blocks ? tiles : blocks), 32 * NWP, smem, s>>>(b);
+    return launch_pdl(kern, dim3((unsigned)(tiles < blocks ? tiles : blocks)), dim3(32 * NWP), smem, s, b);
   }
-  return cudaGetLastError();
 }
 
 template <int R, int MAXG>

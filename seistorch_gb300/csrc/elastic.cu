@@ -105,6 +105,11 @@ struct RowIO {
     if (L.ld && z >= 0 && z < nz) return __ldg(reinterpret_cast<const float4*>(p + (long long)z * pitch + L.xl));
     return f4(0.f);
   }
+  // a row of a field that the launches before this one write
+  __device__ __forceinline__ float4 ldfield(const float* p, int z, const ElLane& L) const {
+    if (L.ld && z >= 0 && z < nz) return ldf4(p + (long long)z * pitch + L.xl);
+    return f4(0.f);
+  }
   __device__ __forceinline__ void st(float* p, int z, const ElLane& L, const float4& v) const {
     if (L.own) *reinterpret_cast<float4*>(p + (long long)z * pitch + L.xl) = v;
   }
@@ -223,6 +228,8 @@ __global__ void __launch_bounds__(128) elastic_fwd_kernel(const ElFwdArgs a) {
   float* sbuf = sbuf_all[threadIdx.x >> 5];
   float* pre = &pre_all[threadIdx.x >> 5][0][0][0];
   const int gw = blockIdx.x * 4 + (threadIdx.x >> 5);
+  pdl_wait();
+  pdl_trigger();
   if (gw >= a.nshots * a.nstrip * a.nband) return;  // whole warps; no block barrier below
   const int b = gw % a.nshots;
   const int rest = gw / a.nshots;
@@ -248,20 +255,20 @@ __global__ void __launch_bounds__(128) elastic_fwd_kernel(const ElFwdArgs a) {
   }
 
   // prologue: rows z0 - 1 and z0
-  const float4 vx_m = io.ld(vx, z0 - 1, L), vz_m = io.ld(vz, z0 - 1, L);
-  float4 vx_c = io.ld(vx, z0, L), vz_c = io.ld(vz, z0, L);
+  const float4 vx_m = io.ldfield(vx, z0 - 1, L), vz_m = io.ldfield(vz, z0 - 1, L);
+  float4 vx_c = io.ldfield(vx, z0, L), vz_c = io.ldfield(vz, z0, L);
   float4 tzz_p = f4(0.f);  // tzz' of row z - 1 (before sources)
   if (z0 >= 1) {
     const float4 E = dxm(vx_m, L), F = vz_c - vz_m;
     const float4 q = io.ld(a.c.q, z0 - 1, L), pa = io.ld(a.c.pa, z0 - 1, L), la = io.ld(a.c.la, z0 - 1, L);
-    tzz_p = fma4(pa, F, fma4(la, E, q * io.ld(tzz, z0 - 1, L)));
+    tzz_p = fma4(pa, F, fma4(la, E, q * io.ldfield(tzz, z0 - 1, L)));
   }
   float4 q_c = io.ld(a.c.q, z0, L), pa_c = io.ld(a.c.pa, z0, L), la_c = io.ld(a.c.la, z0, L);
   float4 bv_c = io.ld(a.c.bv, z0, L);
   float4 txz_c;  // txz' of row z (before sources)
   {
     const float4 G = dxp(vz_c, L) + (z0 >= 1 ? vx_c - vx_m : f4(0.f));
-    txz_c = fma4(io.ld(a.c.ma, z0, L), G, q_c * io.ld(txz, z0, L));
+    txz_c = fma4(io.ld(a.c.ma, z0, L), G, q_c * io.ldfield(txz, z0, L));
   }
 
   auto cp_row = [&](float* dst, const float* src, int zz) {
@@ -385,6 +392,8 @@ __global__ void __launch_bounds__(128) elastic_bwd_kernel(const ElBwdArgs a) {
   float* sbuf = sbuf_all[threadIdx.x >> 5];
   float* pre = bwd_pre + (threadIdx.x >> 5) * 2 * BWD_PRE_ROWS * 128;
   const int gw = blockIdx.x * 4 + (threadIdx.x >> 5);
+  pdl_wait();
+  pdl_trigger();
   if (gw >= a.nshots * a.nstrip * a.nband) return;
   const int b = gw % a.nshots;
   const int rest = gw / a.nshots;
@@ -429,8 +438,8 @@ __global__ void __launch_bounds__(128) elastic_bwd_kernel(const ElBwdArgs a) {
     }
     return v;
   };
-  auto lds = [&](int f, int z) { return fix_s(io.ld(S[f], z, L), f, z); };
-  auto lda = [&](int f, int z) { return fix_a(io.ld(A[f], z, L), f, z); };
+  auto lds = [&](int f, int z) { return fix_s(io.ldfield(S[f], z, L), f, z); };
+  auto lda = [&](int f, int z) { return fix_a(io.ldfield(A[f], z, L), f, z); };
   auto cp_row = [&](float* dst, const float* src, int zz) {
     const bool ok = L.ld && zz >= 0 && zz < nz;
     cp_async16(dst + 4 * L.lane, ok ? src + (long long)zz * a.pitch + L.xl : src, ok ? 16 : 0);
@@ -685,8 +694,7 @@ cudaError_t launch_elastic_fwd(const ElFwdArgs& a0, cudaStream_t s) {
   ElFwdArgs a = a0;
   a.nband = (a.nz + EL_TZ_FWD - 1) / EL_TZ_FWD;
   const long long warps = (long long)a.nshots * a.nstrip * a.nband;
-  elastic_fwd_kernel<EL_TZ_FWD><<<(unsigned)((warps + 3) / 4), 128, 0, s>>>(a);
-  return cudaGetLastError();
+  return launch_pdl(elastic_fwd_kernel<EL_TZ_FWD>, dim3((unsigned)((warps + 3) / 4)), dim3(128), 0, s, a);
 }
 
 cudaError_t launch_elastic_bwd(const ElBwdArgs& a0, int mode, cudaStream_t s) {
@@ -704,11 +712,9 @@ cudaError_t launch_elastic_bwd(const ElBwdArgs& a0, int mode, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     set = true;
   }
-  if (mode == 0)
-    elastic_bwd_kernel<EL_TZ_REV, 0><<<(unsigned)((warps + 3) / 4), 128, smem0, s>>>(a);
-  else
-    elastic_bwd_kernel<EL_TZ_REV, 1><<<(unsigned)((warps + 3) / 4), 128, smem1, s>>>(a);
-  return cudaGetLastError();
+  const dim3 grid((unsigned)((warps + 3) / 4));
+  return mode == 0 ? launch_pdl(elastic_bwd_kernel<EL_TZ_REV, 0>, grid, dim3(128), smem0, s, a)
+                   : launch_pdl(elastic_bwd_kernel<EL_TZ_REV, 1>, grid, dim3(128), smem1, s, a);
 }
 
 cudaError_t launch_elastic_coef(const sgb_grid& g, const float* vp, const float* vs, const float* rho,

@@ -470,10 +470,10 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a) {
     if (c < NST && zs >= 0 && zs < a.nz && xs >= 0 && xs < a.nx) {
       const long long os = (long long)zs * a.pitch + xs;
       g.k = __ldg(reinterpret_cast<const float4*>(kp + os));
-      g.l = *reinterpret_cast<const float4*>(l1 + os);
+      g.l = ldf4(l1 + os);
       if (VTI) g.q = __ldg(reinterpret_cast<const float4*>(a.kz + os));
-      g.v = *reinterpret_cast<const float4*>(u1 + os);
-      if (NEAR) g.m = *reinterpret_cast<const float4*>(a.la2 + fb + os);
+      g.v = ldf4(u1 + os);
+      if (NEAR) g.m = ldf4(a.la2 + fb + os);
       if (NEAR) g.w = wi4_at(zs, xs);
     }
   };
@@ -513,14 +513,14 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a) {
     k4 = __ldg(reinterpret_cast<const float4*>(kp + o));
     if (VTI) kz4 = __ldg(reinterpret_cast<const float4*>(a.kz + o));
     if (!NEAR) {
-      l2g = *reinterpret_cast<const float4*>(a.la2 + fb + o);
-      l1g = *reinterpret_cast<const float4*>(l1 + o);
+      l2g = ldf4(a.la2 + fb + o);
+      l1g = ldf4(l1 + o);
     }
   };
   // U_j of the four cells (reconstruction)
   auto tail_loads = [&]() {
     if (!cell_in) return;
-    if (a.uout != nullptr && row_in) uj4 = *reinterpret_cast<const float4*>(a.uj + fb + o);
+    if (a.uout != nullptr && row_in) uj4 = ldf4(a.uj + fb + o);
   };
   if constexpr (PRE) {
     Grp g[NIT];
@@ -607,7 +607,7 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a) {
         if (ws != 0.f) {
           const long long oo = (long long)pz * a.pitch + px;
           const float c = __ldg(a.vp + oo);
-          acc -= ws * c * c * a.muf * l1[oo];
+          acc -= ws * c * c * a.muf * ldf(l1 + oo);
         }
       }
     }
@@ -661,7 +661,7 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a) {
       if (pz >= 0 && pz < a.nz) {
         const float4 ws = share4(sd, pz);
         coefs(pz, lam, mu);
-        const float4 lw = *reinterpret_cast<const float4*>(l1 + (long long)pz * a.pitch + x);
+        const float4 lw = ldf4(l1 + (long long)pz * a.pitch + x);
 #pragma unroll
         for (int m = 0; m < 4; ++m) set_comp(acc, m, comp(acc, m) - comp(ws, m) * comp(mu, m) * comp(lw, m));
       }
@@ -861,14 +861,27 @@ constexpr int habc_bwd_min_blocks() {
   if (EQ == 2) return 3;
   return R <= 2 ? 3 : 2;
 }
+// The far launch waits for the step before it; the near launch (other cells,
+// nothing of the far launch is read) starts as soon as the far CTAs have all
+// passed that wait, fills the SMs that the far launch's last wave leaves idle,
+// and waits for the far launch only before it ends, so that its completion,
+// which the next step's far launch waits for, is that of the whole step.
+// Without far tiles the near launch waits for the step before it itself.
+template <int R, int EQ, bool NEAR>
+__device__ __forceinline__ void habc_bwd_step(const HabcBwdArgs& a) {
+  if (!NEAR || a.fx1 <= a.fx0) pdl_wait();
+  pdl_trigger();
+  habc_bwd_tile<R, EQ, NEAR>(a);
+  if (NEAR) pdl_wait();
+}
 template <int R, int EQ, bool NEAR>
 __global__ void __launch_bounds__(256) habc_bwd_tile_kernel(const HabcBwdArgs a) {
-  habc_bwd_tile<R, EQ, NEAR>(a);
+  habc_bwd_step<R, EQ, NEAR>(a);
 }
 template <int R, int EQ, bool NEAR>
 __global__ void __launch_bounds__(256, habc_bwd_min_blocks<R, EQ, NEAR>()) habc_bwd_tile_kernel_held(
     const HabcBwdArgs a) {
-  habc_bwd_tile<R, EQ, NEAR>(a);
+  habc_bwd_step<R, EQ, NEAR>(a);
 }
 
 
@@ -977,14 +990,15 @@ cudaError_t launch_habc_bwd(const sgb_grid& g, const sgb_acoustic_model& m, cons
   const dim3 gfar((unsigned)(a.fx1 - a.fx0), (unsigned)(a.fz1 - a.fz0), (unsigned)g.nshots);
   const dim3 gnear((unsigned)nnear, 1u, (unsigned)g.nshots);
   // one launch for the tiles out of reach of the strips, one for the rest
+  cudaError_t err = cudaSuccess;
   switch (R * 3 + eq) {
 #define SGB_TILE2(RR, EQ)                                                                           \
   if constexpr (EQ == 0) {                                                                        \
-    if (nfar > 0) habc_bwd_tile_kernel<RR, EQ, false><<<gfar, dim3(32, HT_Z), 0, s>>>(a);         \
-    if (nnear > 0) habc_bwd_tile_kernel<RR, EQ, true><<<gnear, dim3(32, HT_Z), 0, s>>>(a);        \
+    if (nfar > 0 && err == cudaSuccess) err = launch_pdl(habc_bwd_tile_kernel<RR, EQ, false>, gfar, dim3(32, HT_Z), 0, s, a);         \
+    if (nnear > 0 && err == cudaSuccess) err = launch_pdl(habc_bwd_tile_kernel<RR, EQ, true>, gnear, dim3(32, HT_Z), 0, s, a);        \
   } else {                                                                                        \
-    if (nfar > 0) habc_bwd_tile_kernel_held<RR, EQ, false><<<gfar, dim3(32, HT_Z), 0, s>>>(a);    \
-    if (nnear > 0) habc_bwd_tile_kernel_held<RR, EQ, true><<<gnear, dim3(32, HT_Z), 0, s>>>(a);   \
+    if (nfar > 0 && err == cudaSuccess) err = launch_pdl(habc_bwd_tile_kernel_held<RR, EQ, false>, gfar, dim3(32, HT_Z), 0, s, a);    \
+    if (nnear > 0 && err == cudaSuccess) err = launch_pdl(habc_bwd_tile_kernel_held<RR, EQ, true>, gnear, dim3(32, HT_Z), 0, s, a);   \
   }
     case 3: SGB_TILE2(1, 0) break;
     case 4: SGB_TILE2(1, 1) break;
@@ -998,7 +1012,7 @@ cudaError_t launch_habc_bwd(const sgb_grid& g, const sgb_acoustic_model& m, cons
 #undef SGB_TILE2
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
+  return err;
 }
 
 cudaError_t launch_habc_step_vjp(const sgb_grid& g, const sgb_acoustic_model& m, const sgb_habc_vjp_io& io,
