@@ -69,7 +69,8 @@ cudaError_t launch_acoustic_fwd_stream(int R, const CUtensorMap* maps, const AcS
                                        bool habc = false);
 int habc_tile_rows(int R, int hb);
 int vacoustic_kterm(const sgb_grid& g, const float* pre, const float* u1, const float* u2, const float* post,
-                    float* out, float* work, float* tw, cudaStream_t s);
+                    float* out, float* work, float* tw, cudaStream_t s, bool tables = true);
+int64_t vacoustic_table_floats(const sgb_grid& g);
 
 // Viscoacoustic extras of a forward loop: before each step the damping term
 // extra = a_neg * K(U_n - U_{n-1}) is formed and added to the interior
@@ -398,7 +399,7 @@ int sgb_vacoustic_work_size(const sgb_grid* grid, int64_t* work_floats, int64_t*
   if (int e = check_grid(grid)) return e;
   if (work_floats == nullptr || tw_floats == nullptr) return SGB_ERR_ARG;
   *work_floats = 2LL * ((grid->nshots + 1) / 2) * grid->nz * grid->nx;
-  *tw_floats = 2LL * (grid->nz + grid->nx);
+  *tw_floats = vacoustic_table_floats(*grid);
   return SGB_OK;
 }
 
@@ -521,7 +522,8 @@ int acoustic_forward_impl(const sgb_grid* grid, const sgb_acoustic_model* model,
                                             : nullptr;
     const CUtensorMap maps[2] = {mu[cur], mum[prev]};
     if (vac != nullptr) {
-      if (int e = vacoustic_kterm(*grid, nullptr, buf[cur], buf[prev], vac->a_neg, vac->extra, vac->work, vac->tw, s))
+      if (int e = vacoustic_kterm(*grid, nullptr, buf[cur], buf[prev], vac->a_neg, vac->extra, vac->work, vac->tw, s,
+                                  t == 0))
         return e;
       sa.born_in = vac->extra;
     }
