@@ -600,6 +600,17 @@ typedef struct {
 } sgb_nn_wgrad;
 int sgb_nn_conv3x3_wgrad(const sgb_nn_wgrad *p, sgb_stream_t stream);
 
+/* The same from the NHWC tensors themselves (no transposed copies): dy bf16
+ * [n][h][w][cout], x bf16 [n][h][w][cin], both 16-byte aligned, w a multiple of
+ * 64, channels multiples of 8; dw as above (accumulated). */
+typedef struct {
+  int32_t n, h, w, cin, cout;
+  const void *dy;
+  const void *x;
+  float *dw;
+} sgb_nn_wgrad_nhwc;
+int sgb_nn_conv3x3_wgrad_nhwc(const sgb_nn_wgrad_nhwc *p, sgb_stream_t stream);
+
 /* NHWC (channel slice [coff, coff + c) of a tensor with cstride channels)
  * -> CHW bf16 [copies][n][c][h][w]: copies = 1 gives the plain transpose,
  * copies = 3 the three column-shifted copies sgb_nn_conv3x3_wgrad reads. */
@@ -636,6 +647,8 @@ int sgb_nn_up2_bwd(int32_t n, int32_t h, int32_t w, int32_t c, const float *g, i
 int sgb_nn_pool2_bwd(int32_t n, int32_t h, int32_t w, int32_t c, const float *gp, const float *gs, int32_t cs_s,
                      int32_t coff_s, const void *act, int32_t cs_a, int32_t coff_a, void *out, sgb_stream_t stream);
 int sgb_nn_bias_grad(int32_t n, int64_t hw, int32_t c, const void *dy_chw, float *db, sgb_stream_t stream);
+/* db[c] += sum over pixels of dy[pixel][c] (bf16, c a multiple of 8, 16-byte aligned) */
+int sgb_nn_bias_grad_nhwc(int64_t pixels, int32_t c, const void *dy, float *db, sgb_stream_t stream);
 int sgb_nn_pack_weights(int32_t cout, int32_t cin, const float *W, void *wt, void *wflip, sgb_stream_t stream);
 int sgb_nn_adam(int64_t n, float *p, const float *g, float *m, float *v, float lr, float b1, float b2, float eps,
                 int32_t step, float wd, sgb_stream_t stream);

@@ -21,7 +21,7 @@ LIB_NAME = "libseistorch_gb300.so"
 LIB_PATH = os.path.join(BUILD_DIR, LIB_NAME)
 SOURCES = ["acoustic.cu", "acoustic_stream.cu", "acoustic_stream_fwd.cu", "acoustic_stream_bwd.cu",
            "elastic.cu", "capi.cu", "capi_elastic.cu", "capi_batch.cu", "noalloc.cu",
-           "nn_gemm.cu", "nn_ops.cu", "capi_nn.cu", "habc_bwd.cu", "postproc.cu", "fft.cu"]
+           "nn_gemm.cu", "nn_wgrad.cu", "nn_ops.cu", "capi_nn.cu", "habc_bwd.cu", "postproc.cu", "fft.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 
@@ -128,6 +128,11 @@ class NnWgrad(ctypes.Structure):
                 ("dy_chw", c_ptr), ("x_chw", c_ptr * 3), ("dw", c_ptr)]
 
 
+class NnWgradNhwc(ctypes.Structure):
+    _fields_ = [("n", c_i32), ("h", c_i32), ("w", c_i32), ("cin", c_i32), ("cout", c_i32),
+                ("dy", c_ptr), ("x", c_ptr), ("dw", c_ptr)]
+
+
 PTR3 = c_ptr * 3
 PTR2 = c_ptr * 2
 PTR5 = c_ptr * 5
@@ -190,6 +195,8 @@ SIGNATURES = {
     "sgb_plan_destroy": (ctypes.c_int, [c_ptr]),
     "sgb_nn_conv3x3": (ctypes.c_int, [ctypes.POINTER(NnConv), c_ptr]),
     "sgb_nn_conv3x3_wgrad": (ctypes.c_int, [ctypes.POINTER(NnWgrad), c_ptr]),
+    "sgb_nn_conv3x3_wgrad_nhwc": (ctypes.c_int, [ctypes.POINTER(NnWgradNhwc), c_ptr]),
+    "sgb_nn_bias_grad_nhwc": (ctypes.c_int, [ctypes.c_int64, c_i32, c_ptr, c_ptr, c_ptr]),
     "sgb_nn_to_chw": (ctypes.c_int, [c_i32, c_i32, c_i32, c_i32, c_i32, c_i32, c_ptr, c_i32, c_ptr, c_ptr]),
     "sgb_nn_conv_in": (ctypes.c_int, [c_i32, c_i32, c_i32, c_i32, c_ptr, c_ptr, c_ptr, c_ptr, c_i32, c_i32, c_ptr]),
     "sgb_nn_conv_in_wgrad": (ctypes.c_int, [c_i32, c_i32, c_i32, c_i32, c_ptr, c_ptr, c_i32, c_ptr, c_ptr,

@@ -11,7 +11,10 @@
 namespace sgb {
 namespace nn {
 cudaError_t launch_gemm(int bn, int rb, const CUtensorMap* maps, const GemmArgs& g, dim3 grid, cudaStream_t s);
+cudaError_t launch_wgrad(const CUtensorMap* maps, const WgradArgs& g, cudaStream_t s);
+int wgrad_bn(const WgradArgs& g);
 using bf16 = __nv_bfloat16;
+cudaError_t launch_bias_grad_nhwc(long long pixels, int c, const bf16* dy, float* db, cudaStream_t s);
 cudaError_t launch_to_chw(int n, int h, int w, int c, int cstride, int coff, const bf16* x, int copies, bf16* out,
                           cudaStream_t s);
 cudaError_t launch_conv_in_fwd(int n, int h, int w, int c, const float* in, const float* W, const float* b, bf16* out,
@@ -192,6 +195,37 @@ int sgb_nn_conv3x3_wgrad(const sgb_nn_wgrad* p, sgb_stream_t stream) {
   return SGB_OK;
 }
 
+int sgb_nn_conv3x3_wgrad_nhwc(const sgb_nn_wgrad_nhwc* p, sgb_stream_t stream) {
+  if (p == nullptr || p->dy == nullptr || p->x == nullptr || p->dw == nullptr) return SGB_ERR_ARG;
+  if (p->n <= 0 || p->h <= 0 || p->cin <= 0 || p->cout <= 0 || p->w <= 0 || p->w % 64 != 0) return SGB_ERR_SHAPE;
+  if (p->cin % 8 != 0 || p->cout % 8 != 0) return SGB_ERR_SHAPE;
+  if (!aligned16(p->dy) || !aligned16(p->x)) return SGB_ERR_ALIGN;
+  WgradArgs g;
+  std::memset(&g, 0, sizeof(g));
+  g.N = p->n;
+  g.H = p->h;
+  g.W = p->w;
+  g.Cin = p->cin;
+  g.Cout = p->cout;
+  g.wchunks = p->w / 64;
+  g.kiters = p->n * p->h * g.wchunks;
+  g.dw = p->dw;
+  g.status = status_ptr();
+  const int bn = wgrad_bn(g);
+  CUtensorMap maps[2];
+  const void* ptr[2] = {p->x, p->dy};
+  for (int k = 0; k < 2; ++k) {
+    const uint64_t c = k == 0 ? p->cin : p->cout, eb = 2;
+    const int rb = (k == 0 || bn >= 64) ? 128 : 64;
+    const uint64_t dims[4] = {c, (uint64_t)p->w, (uint64_t)p->h, (uint64_t)p->n};
+    const uint64_t st[3] = {c * eb, p->w * c * eb, (uint64_t)p->h * p->w * c * eb};
+    const uint32_t box[4] = {(uint32_t)rb / 2, k == 0 ? 66u : 64u, 1, 1};
+    if (bf16_map(&maps[k], ptr[k], 4, dims, st, box, rb)) return SGB_ERR_CUDA;
+  }
+  SGB_CUDA_CHECK(launch_wgrad(maps, g, (cudaStream_t)stream));
+  return SGB_OK;
+}
+
 int sgb_nn_to_chw(int32_t n, int32_t h, int32_t w, int32_t c, int32_t cstride, int32_t coff, const void* x_nhwc,
                   int32_t copies, void* out, sgb_stream_t stream) {
   if (x_nhwc == nullptr || out == nullptr || (copies != 1 && copies != 3)) return SGB_ERR_ARG;
@@ -284,6 +318,14 @@ int sgb_nn_bias_grad(int32_t n, int64_t hw, int32_t c, const void* dy_chw, float
   if (dy_chw == nullptr || db == nullptr) return SGB_ERR_ARG;
   if (n <= 0 || hw <= 0 || c <= 0) return SGB_ERR_SHAPE;
   SGB_CUDA_CHECK(launch_bias_grad(n, hw, c, BF(dy_chw), db, (cudaStream_t)stream));
+  return SGB_OK;
+}
+
+int sgb_nn_bias_grad_nhwc(int64_t pixels, int32_t c, const void* dy, float* db, sgb_stream_t stream) {
+  if (dy == nullptr || db == nullptr) return SGB_ERR_ARG;
+  if (pixels <= 0 || c <= 0 || c % 8) return SGB_ERR_SHAPE;
+  if (!aligned16(dy)) return SGB_ERR_ALIGN;
+  SGB_CUDA_CHECK(launch_bias_grad_nhwc(pixels, c, BF(dy), db, (cudaStream_t)stream));
   return SGB_OK;
 }
 

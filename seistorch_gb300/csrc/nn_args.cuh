@@ -33,5 +33,15 @@ struct GemmArgs {
   int gx, gy, gz;
 };
 
+// Weight gradient from NHWC operands (nn_wgrad.cu).
+struct WgradArgs {
+  int N, H, W, Cin, Cout;
+  int wchunks;      // W / 64
+  int kiters;       // N * H * wchunks
+  int k_per_split;  // K steps per CTA
+  float* dw;        // [Cout][Cin][3][3], accumulated
+  int* status;
+};
+
 }  // namespace nn
 }  // namespace sgb

@@ -32,20 +32,12 @@
 
 #include "sgb_common.cuh"
 #include "tma.cuh"
+#include "tcgen05.cuh"
 #include "nn_args.cuh"
 
 namespace sgb {
 namespace nn {
 namespace {
-
-__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
-                                            uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
-      : "memory");
-}
 
 // Shared-memory matrix descriptor of a K-major, swizzled operand tile whose
 // rows are RB bytes (RB = 128: 128-byte swizzle, RB = 64: 64-byte swizzle);
@@ -55,46 +47,6 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
   constexpr uint64_t layout = RB == 128 ? 2ull : 4ull;  // SWIZZLE_128B : SWIZZLE_64B
   constexpr uint64_t sbo = (8ull * RB) >> 4;
   return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | (sbo << 32) | (1ull << 46) | (layout << 61);
-}
-
-// Instruction descriptor: D fp32, A and B bf16, both K-major, M = 128, N = BN.
-template <int BN>
-__device__ __forceinline__ uint32_t instr_desc() {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-}
-
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(idesc), "r"(acc)
-      : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                   smem_u32(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-
-// 16 consecutive fp32 columns of this thread's TMEM lane.
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-      "%15}, [%16];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 template <int BN, int RB, int S>
@@ -185,10 +137,7 @@ __global__ void __launch_bounds__(192, 1) nn_gemm_kernel(const __grid_constant__
   const int ntiles = g.gx * g.gy * g.gz;
 
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)),
-                 "r"(Lay::TMEM_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    tmem_alloc(tmem_slot, Lay::TMEM_COLS);
   }
   if (threadIdx.x == 32) {
     for (int s = 0; s < S; ++s) {
@@ -249,7 +198,7 @@ __global__ void __launch_bounds__(192, 1) nn_gemm_kernel(const __grid_constant__
     s_issued = it;
   } else if (warp == 1 && lane == 0) {
     // ---- MMA issuer
-    const uint32_t idesc = instr_desc<BN>();
+    const uint32_t idesc = mma_idesc_bf16(128, BN);
     int it = 0, lt = 0;  // K steps consumed, tiles of this CTA
     for (int t = blockIdx.x; t < ntiles && !*fail; t += gridDim.x, ++lt) {
       const GemmTile q = decode_tile<BN>(g, t);
@@ -393,8 +342,7 @@ __global__ void __launch_bounds__(192, 1) nn_gemm_kernel(const __grid_constant__
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(Lay::TMEM_COLS)
-                 : "memory");
+    tmem_dealloc(tmem, Lay::TMEM_COLS);
   }
 }
 

@@ -117,8 +117,6 @@ class PrecondNet:
             g1=bf(h1, w1, 32), g1b=bf(h1, w1, 32), dcat1=f32(h1, w1, 96), g2=bf(h2, w2, 64), g2b=bf(h2, w2, 64),
             dcat2=f32(h2, w2, 192), g3=bf(h3, w3, 128), g3b=bf(h3, w3, 128), dcat3=f32(h3, w3, 384),
             g4=bf(h4, w4, 256), dp3=f32(h4, w4, 128), dp2=f32(h3, w3, 64), dp1=f32(h2, w2, 32),
-            chw_dy=torch.zeros(B * h1 * w1 * 64, dtype=BF16, device=d),
-            chw_x=torch.zeros(3 * B * h1 * w1 * 96, dtype=BF16, device=d),
             dpred=torch.zeros(B, h1, w1, dtype=torch.float32, device=d),
             loss=torch.zeros(1, dtype=torch.float32, device=d))
         self._bufs, self._shape, self._levels = b, (B, H, W), L
@@ -141,21 +139,11 @@ class PrecondNet:
 
     def _tc_wgrad(self, name, dy, x, h, w):
         _, ci, co, _ = next(l for l in LAYERS if l[0] == name)
-        b = self._bufs
         B = self._shape[0]
         s = N.stream_handle()
-        n_dy = B * co * h * w
-        n_x = B * ci * h * w
-        dy_chw = b["chw_dy"][:n_dy] if n_dy <= b["chw_dy"].numel() else torch.empty(n_dy, dtype=BF16,
-                                                                                     device=self.device)
-        x_chw = b["chw_x"][:3 * n_x] if 3 * n_x <= b["chw_x"].numel() else torch.empty(3 * n_x, dtype=BF16,
-                                                                                        device=self.device)
-        N.call("sgb_nn_to_chw", B, h, w, co, co, 0, N.ptr(dy), 1, N.ptr(dy_chw), s)
-        N.call("sgb_nn_to_chw", B, h, w, ci, ci, 0, N.ptr(x), 3, N.ptr(x_chw), s)
-        p = N.NnWgrad(B, h, w, ci, co, N.ptr(dy_chw),
-                      N.PTR3(*[x_chw.data_ptr() + 2 * k * n_x for k in range(3)]), N.ptr(self.gW[name]))
-        N.call("sgb_nn_conv3x3_wgrad", ctypes.byref(p), s)
-        N.call("sgb_nn_bias_grad", B, h * w, co, N.ptr(dy_chw), N.ptr(self.gb[name]), s)
+        p = N.NnWgradNhwc(B, h, w, ci, co, N.ptr(dy), N.ptr(x), N.ptr(self.gW[name]))
+        N.call("sgb_nn_conv3x3_wgrad_nhwc", ctypes.byref(p), s)
+        N.call("sgb_nn_bias_grad_nhwc", B * h * w, co, N.ptr(dy), N.ptr(self.gb[name]), s)
 
     # -- forward / backward
     def forward(self, x):
