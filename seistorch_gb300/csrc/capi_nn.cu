@@ -11,6 +11,8 @@
 namespace sgb {
 namespace nn {
 cudaError_t launch_gemm(int bn, int rb, const CUtensorMap* maps, const GemmArgs& g, dim3 grid, cudaStream_t s);
+int conv_row_bn(const GemmArgs& g, int rb);
+cudaError_t launch_conv_row(int bn, int rb, const CUtensorMap* maps, const GemmArgs& g, cudaStream_t s);
 cudaError_t launch_wgrad(const CUtensorMap* maps, const WgradArgs& g, cudaStream_t s);
 int wgrad_bn(const WgradArgs& g);
 using bf16 = __nv_bfloat16;
@@ -105,7 +107,6 @@ int sgb_nn_conv3x3(const sgb_nn_conv* c, sgb_stream_t stream) {
     return SGB_ERR_SHAPE;
   if (!aligned16(c->x) || !aligned16(c->wt)) return SGB_ERR_ALIGN;
   const int rb = c->cin % 64 == 0 ? 128 : 64;
-  const int bn = pick_bn(c->cout);
   GemmArgs g;
   std::memset(&g, 0, sizeof(g));
   g.mode = MODE_CONV;
@@ -129,12 +130,14 @@ int sgb_nn_conv3x3(const sgb_nn_conv* c, sgb_stream_t stream) {
   g.out_cstride = c->out_cstride;
   g.out_coff = c->out_coff;
   g.status = status_ptr();
+  const int row_bn = conv_row_bn(g, rb);  // weights and input rows on chip
+  const int bn = row_bn > 0 ? row_bn : pick_bn(c->cout);
   CUtensorMap maps[4];
   const uint64_t eb = 2;
   {
     const uint64_t dims[4] = {(uint64_t)c->cin, (uint64_t)c->w, (uint64_t)c->h, (uint64_t)c->n};
     const uint64_t st[3] = {c->cin * eb, (uint64_t)c->w * c->cin * eb, (uint64_t)c->h * c->w * c->cin * eb};
-    const uint32_t box[4] = {(uint32_t)(rb / 2), (uint32_t)g.TW, (uint32_t)g.TH, 1};
+    const uint32_t box[4] = {(uint32_t)(rb / 2), row_bn > 0 ? 130u : (uint32_t)g.TW, row_bn > 0 ? 1u : (uint32_t)g.TH, 1};
     if (bf16_map(&maps[0], c->x, 4, dims, st, box, rb)) return SGB_ERR_CUDA;
   }
   {
@@ -142,6 +145,10 @@ int sgb_nn_conv3x3(const sgb_nn_conv* c, sgb_stream_t stream) {
     const uint64_t st[2] = {c->cin * eb, 9ull * c->cin * eb};
     const uint32_t box[3] = {(uint32_t)(rb / 2), 1, (uint32_t)bn};
     if (bf16_map(&maps[1], c->wt, 3, dims, st, box, rb)) return SGB_ERR_CUDA;
+  }
+  if (row_bn > 0) {
+    SGB_CUDA_CHECK(launch_conv_row(row_bn, rb, maps, g, (cudaStream_t)stream));
+    return SGB_OK;
   }
   maps[2] = maps[1];
   maps[3] = maps[1];

@@ -32,22 +32,11 @@
 
 #include "sgb_common.cuh"
 #include "tma.cuh"
-#include "tcgen05.cuh"
-#include "nn_args.cuh"
+#include "nn_epilogue.cuh"
 
 namespace sgb {
 namespace nn {
 namespace {
-
-// Shared-memory matrix descriptor of a K-major, swizzled operand tile whose
-// rows are RB bytes (RB = 128: 128-byte swizzle, RB = 64: 64-byte swizzle);
-// 8-row groups are 8 * RB bytes apart.
-template <int RB>
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-  constexpr uint64_t layout = RB == 128 ? 2ull : 4ull;  // SWIZZLE_128B : SWIZZLE_64B
-  constexpr uint64_t sbo = (8ull * RB) >> 4;
-  return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | (sbo << 32) | (1ull << 46) | (layout << 61);
-}
 
 template <int BN, int RB, int S>
 struct GemmLayout {
@@ -87,17 +76,6 @@ __device__ __forceinline__ GemmTile decode_tile(const GemmArgs& g, int t) {
     q.kend = min(q.kbeg + g.k_per_split, g.kiters);
   }
   return q;
-}
-
-// 16-byte store of eight bf16 / four fp32 values
-__device__ __forceinline__ void st_bf16x8(__nv_bfloat16* p, const float* v) {
-  uint32_t w[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-    w[i] = *reinterpret_cast<const uint32_t*>(&h);
-  }
-  *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
 // Persistent CTA of 192 threads walking the tiles t = blockIdx.x,
@@ -250,68 +228,8 @@ __global__ void __launch_bounds__(192, 1) nn_gemm_kernel(const __grid_constant__
       const uint32_t taddr = tmem + (uint32_t)(buf * Lay::ACC_COLS) + ((uint32_t)(quarter * 32) << 16);
       if (g.mode == MODE_CONV) {
         const int py = q.y0 + row / g.TW, px = q.x0 + row % g.TW;
-        const bool inrow = py < g.H && px < g.W;
         const long long pix = ((long long)q.n_img * g.H + py) * g.W + px;
-        const bool vb = ((g.out_cstride | g.out_coff) & 7) == 0;
-        const bool vf = ((g.out_cstride | g.out_coff) & 3) == 0;
-        const bool vm = (g.mask_cstride & 7) == 0;
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 16) {
-          float v[16];
-          tmem_ld16(taddr + c, v);
-          const int co = q.n0 + c;
-          if (!inrow || co >= g.Cout) continue;
-          const bool whole = co + 16 <= g.Cout;
-          if (g.bias != nullptr) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] += (co + j < g.Cout) ? __ldg(g.bias + co + j) : 0.f;
-          }
-          if (g.relu) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = v[j] < 0.f ? 0.f : v[j];
-          }
-          if (g.mask != nullptr) {
-            const __nv_bfloat16* mp = g.mask + pix * g.mask_cstride + co;
-            if (whole && vm) {
-              const uint4 m0 = __ldg(reinterpret_cast<const uint4*>(mp));
-              const uint4 m1 = __ldg(reinterpret_cast<const uint4*>(mp + 8));
-              const __nv_bfloat16* mb0 = reinterpret_cast<const __nv_bfloat16*>(&m0);
-              const __nv_bfloat16* mb1 = reinterpret_cast<const __nv_bfloat16*>(&m1);
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                v[j] = __bfloat162float(mb0[j]) > 0.f ? v[j] : 0.f;
-                v[8 + j] = __bfloat162float(mb1[j]) > 0.f ? v[8 + j] : 0.f;
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 16; ++j)
-                if (co + j < g.Cout) v[j] = __bfloat162float(mp[j]) > 0.f ? v[j] : 0.f;
-            }
-          }
-          if (g.out_f32 != nullptr) {
-            float* o = g.out_f32 + pix * g.out_cstride + g.out_coff + co;
-            if (whole && vf) {
-#pragma unroll
-              for (int j = 0; j < 16; j += 4)
-                *reinterpret_cast<float4*>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-            } else {
-#pragma unroll
-              for (int j = 0; j < 16; ++j)
-                if (co + j < g.Cout) o[j] = v[j];
-            }
-          }
-          if (g.out_bf16 != nullptr) {
-            __nv_bfloat16* o = g.out_bf16 + pix * g.out_cstride + g.out_coff + co;
-            if (whole && vb) {
-              st_bf16x8(o, v);
-              st_bf16x8(o + 8, v + 8);
-            } else {
-#pragma unroll
-              for (int j = 0; j < 16; ++j)
-                if (co + j < g.Cout) o[j] = __float2bfloat16_rn(v[j]);
-            }
-          }
-        }
+        conv_epilogue<BN>(g, taddr, q.n0, pix, py < g.H && px < g.W);
       } else {
         // dW[co][ci][tap] += D[co][ci]   (the [cout][cin][3][3] layout)
 #pragma unroll 1

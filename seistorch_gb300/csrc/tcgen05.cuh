@@ -19,6 +19,16 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, i
       : "memory");
 }
 
+// Shared-memory matrix descriptor of a K-major, swizzled operand tile whose
+// rows are RB bytes (RB = 128: 128-byte swizzle, RB = 64: 64-byte swizzle);
+// 8-row groups are 8 * RB bytes apart.
+template <int RB>
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
+  constexpr uint64_t layout = RB == 128 ? 2ull : 4ull;  // SWIZZLE_128B : SWIZZLE_64B
+  constexpr uint64_t sbo = (8ull * RB) >> 4;
+  return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | (sbo << 32) | (1ull << 46) | (layout << 61);
+}
+
 // Instruction descriptor: D fp32, A and B bf16, both K-major (bits 15 / 16: A / B MN-major).
 __device__ __forceinline__ uint32_t mma_idesc_bf16(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);

@@ -104,3 +104,28 @@ def test_weight_gradient_matches_torch(N, n, h, w, cin, cout):
     torch.cuda.synchronize()
     assert rel_l2(dw.cpu().numpy(), want.cpu().numpy()) < 2e-3
     assert N.device_status() == 0
+
+
+@pytest.mark.parametrize("n,h,w,cin,cout", [(1, 608, 128, 32, 32), (2, 160, 256, 96, 32), (1, 305, 256, 64, 64),
+                                            (3, 230, 128, 32, 96), (1, 700, 128, 64, 40), (1, 620, 128, 96, 24)])
+def test_rows_on_chip_convolution(N, n, h, w, cin, cout):
+    """The kernel that keeps weights and input rows on chip (images of at
+    least 608 rows of 128 pixels): strips that end inside a CTA's range, output
+    channels below and at the tile, fp32 with mask and a channel slice, bf16
+    with bias and ReLU.  fp32 sums of 9 cin bf16 products: 1e-5."""
+    torch.manual_seed(h + cin)
+    dev = torch.device("cuda:0")
+    x = torch.randn(n, cin, h, w, device=dev).bfloat16().float()
+    wt = (torch.randn(cout, cin, 3, 3, device=dev) / (3 * cin ** 0.5)).bfloat16().float()
+    bias = torch.randn(cout, device=dev)
+    xn, w9 = x.permute(0, 2, 3, 1).contiguous().bfloat16(), _w9(wt).bfloat16()
+    want = F.conv2d(x.double(), wt.double(), padding=1).permute(0, 2, 3, 1)
+    mask = torch.randn(n, h, w, cout, device=dev).bfloat16()
+    out = torch.full((n, h, w, cout + 16), 7.0, device=dev)
+    _conv(N, xn, w9, mask=mask, out_f32=out, cstride=cout + 16, coff=8)
+    assert rel_l2(out[..., 8:-8].cpu().numpy(), (want * (mask > 0)).cpu().numpy()) < 1e-5
+    assert torch.all(out[..., :8] == 7.0) and torch.all(out[..., -8:] == 7.0)
+    outb = torch.empty(n, h, w, cout, device=dev, dtype=torch.bfloat16)
+    _conv(N, xn, w9, bias, True, out_bf16=outb)
+    assert rel_l2(outb.float().cpu().numpy(), F.relu(want + bias.double()).cpu().numpy()) < 4e-3
+    assert N.device_status() == 0
