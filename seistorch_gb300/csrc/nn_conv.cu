@@ -109,44 +109,49 @@ __global__ void __launch_bounds__(192) nn_conv_row_kernel(const __grid_constant_
       }
     }
     s_issued = r;
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
+    const uint32_t el = elect_one();
     const uint32_t idesc = mma_idesc_bf16(128, BN);
     const uint32_t wbase = smem_u32(base), rbase = smem_u32(rows);
     int r = 0;  // rows waited for
-    bool ok = mbar_wait(wfull, 0, g.status);
-    for (int t = t0, lt = 0; t < t1 && ok && !*fail; ++t, ++lt) {
+    // every decision is warp-uniform: the MMAs are issued by one lane of a converged warp
+    auto wait = [&](uint64_t* bar, int parity) -> bool {
+      return __all_sync(0xffffffffu, !*fail && mbar_wait(bar, parity, g.status));
+    };
+    bool ok = wait(wfull, 0);
+    for (int t = t0, lt = 0; t < t1 && ok; ++t, ++lt) {
       const int y = t % g.H, buf = lt & 1;
       const int need = (t == t0 || y == 0) ? 3 : 1;
-      for (int i = 0; i < need && ok; ++i, ++r) ok = mbar_wait(&full[r % R], (r / R) & 1, g.status);
-      if (ok && lt >= 2) ok = mbar_wait(&acc_empty[buf], ((lt >> 1) - 1) & 1, g.status);
+      for (int i = 0; i < need && ok; ++i, ++r) ok = wait(&full[r % R], (r / R) & 1);
+      if (ok && lt >= 2) ok = wait(&acc_empty[buf], ((lt >> 1) - 1) & 1);
       if (!ok) break;
       tc_fence_after();
       const uint32_t d = tmem + (uint32_t)(buf * Lay::ACC);
-      uint32_t on = 0;
       for (int ky = 0; ky < 3; ++ky) {
-        const uint32_t row = rbase + (uint32_t)(((r - 3 + ky) % R) * slot_bytes);
+        const uint64_t da0 = smem_desc<RB>(rbase + (uint32_t)(((r - 3 + ky) % R) * slot_bytes));
+        const uint64_t db0 = smem_desc<RB>(wbase + (uint32_t)(ky * 3 * g.nchunk * Lay::W_PANEL));
+#pragma unroll
         for (int kx = 0; kx < 3; ++kx)
           for (int c = 0; c < g.nchunk; ++c) {
-            const uint64_t da = smem_desc<RB>(row + c * Lay::PANEL + kx * RB);
-            const uint64_t db = smem_desc<RB>(wbase + ((ky * 3 + kx) * g.nchunk + c) * Lay::W_PANEL);
+            const uint64_t da = da0 + (uint64_t)((c * Lay::PANEL + kx * RB) >> 4);
+            const uint64_t db = db0 + (uint64_t)(((kx * g.nchunk + c) * Lay::W_PANEL) >> 4);
 #pragma unroll
-            for (int kk = 0; kk < KSTEPS; ++kk) {
-              mma_bf16(d, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), idesc, on);
-              on = 1;
-            }
+            for (int kk = 0; kk < KSTEPS; ++kk)
+              mma_bf16(el, d, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), idesc,
+                       (kx > 0 || kk > 0) ? 1u : (uint32_t)(ky + c));
           }
       }
       // the row above is done with; the strip's last tile is done with all three
-      mma_commit(&empty[(r - 3) % R]);
+      mma_commit(el, &empty[(r - 3) % R]);
       if (y == g.H - 1) {
-        mma_commit(&empty[(r - 2) % R]);
-        mma_commit(&empty[(r - 1) % R]);
+        mma_commit(el, &empty[(r - 2) % R]);
+        mma_commit(el, &empty[(r - 1) % R]);
       }
-      mma_commit(&acc_full[buf]);
+      mma_commit(el, &acc_full[buf]);
     }
     if (!ok) *fail = 1;
-    s_consumed = r;
-    mma_commit(done);  // completes once every MMA issued above has finished
+    if (lane == 0) s_consumed = r;
+    mma_commit(el, done);  // completes once every MMA issued above has finished
   } else if (warp >= 2) {
     const int quarter = warp & 3;  // TMEM lanes 32 (warp % 4) .. + 31
     for (int t = t0, lt = 0; t < t1; ++t, ++lt) {

@@ -6,7 +6,7 @@
 //   warp 0 lane 0  -- TMA producer: per K step one A box (128 rows x RB
 //                     bytes) and one B box (BN rows x RB bytes) into a stage
 //                     of an S-deep ring, 128/64-byte swizzled;
-//   warp 1 lane 0  -- MMA issuer: RB/32 tcgen05.mma (K = 16) per stage, then
+//   warp 1         -- MMA issuer (one elected lane): RB/32 tcgen05.mma (K = 16) per stage, then
 //                     tcgen05.commit to the stage's "empty" mbarrier;
 //   all 4 warps    -- epilogue: tcgen05.ld of their 32 TMEM lanes (= rows).
 // Warp 0 allocates and frees the TMEM columns.  Every wait is bounded; on a
@@ -83,7 +83,7 @@ __device__ __forceinline__ GemmTile decode_tile(const GemmArgs& g, int t) {
 //   warp 0 lane 0  -- TMA producer: per K step one A box (128 rows x RB
 //                     bytes) and one B box (BN rows x RB bytes) into the next
 //                     stage of an S-deep ring that runs on across tiles;
-//   warp 1 lane 0  -- MMA issuer: RB/32 tcgen05.mma (K = 16) per stage into
+//   warp 1         -- MMA issuer (one elected lane): RB/32 tcgen05.mma (K = 16) per stage into
 //                     accumulator buffer (tile & 1), tcgen05.commit to the
 //                     stage's "empty" barrier and, after a tile's last stage,
 //                     to the buffer's "full" barrier;
@@ -174,23 +174,27 @@ __global__ void __launch_bounds__(192, 1) nn_gemm_kernel(const __grid_constant__
       }
     }
     s_issued = it;
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
     // ---- MMA issuer
+    const uint32_t el = elect_one();
     const uint32_t idesc = mma_idesc_bf16(128, BN);
     int it = 0, lt = 0;  // K steps consumed, tiles of this CTA
-    for (int t = blockIdx.x; t < ntiles && !*fail; t += gridDim.x, ++lt) {
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++lt) {
       const GemmTile q = decode_tile<BN>(g, t);
       if (q.kend <= q.kbeg) continue;  // (no such tile: every split has a step)
       const int buf = lt & 1;
-      if (lt >= 2 && !mbar_wait(&acc_empty[buf], ((lt >> 1) - 1) & 1, g.status)) {
+      // every decision is warp-uniform: one lane of a converged warp issues
+      if (!__all_sync(0xffffffffu, !*fail && (lt < 2 || mbar_wait(&acc_empty[buf], ((lt >> 1) - 1) & 1, g.status)))) {
         *fail = 1;
         break;
       }
+      bool ok = true;
       tc_fence_after();
       const uint32_t d = tmem + (uint32_t)(buf * Lay::ACC_COLS);
       for (int k = q.kbeg; k < q.kend; ++k) {
         const int s = it % S;
-        if (!mbar_wait(&full[s], (it / S) & 1, g.status)) {
+        ok = __all_sync(0xffffffffu, !*fail && mbar_wait(&full[s], (it / S) & 1, g.status));
+        if (!ok) {
           *fail = 1;
           break;
         }
@@ -200,15 +204,15 @@ __global__ void __launch_bounds__(192, 1) nn_gemm_kernel(const __grid_constant__
         const uint64_t da = smem_desc<RB>(sa), db = smem_desc<RB>(sb);
 #pragma unroll
         for (int kk = 0; kk < KSTEPS; ++kk)
-          mma_bf16(d, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), idesc, (k > q.kbeg || kk > 0) ? 1u : 0u);
-        mma_commit(&empty[s]);
+          mma_bf16(el, d, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), idesc, (k > q.kbeg || kk > 0) ? 1u : 0u);
+        mma_commit(el, &empty[s]);
         ++it;
       }
-      if (*fail) break;
-      mma_commit(&acc_full[buf]);
+      if (!ok) break;
+      mma_commit(el, &acc_full[buf]);
     }
-    s_consumed = it;
-    mma_commit(done);  // completes once every MMA issued above has finished
+    if (lane == 0) s_consumed = it;
+    mma_commit(el, done);  // completes once every MMA issued above has finished
   } else if (warp >= 2) {
     // ---- epilogue
     const int quarter = warp & 3;

@@ -110,12 +110,14 @@ __global__ void __launch_bounds__(128) nn_wgrad_kernel(const __grid_constant__ C
         tma_load_4d(sb + p * Lay::B_PANEL, &tmD, n0 + 64 * p, xc * WG_PX, y, n, &full[s]);
     }
     s_issued = it;
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
+    const uint32_t el = elect_one();
     const uint32_t idesc = mma_idesc_bf16(128, BN) | (1u << 15) | (1u << 16);  // A and B MN-major
     int it = 0;
-    for (int k = k0; k < k1 && !*fail; ++k, ++it) {
+    for (int k = k0; k < k1; ++k, ++it) {
       const int s = it % S;
-      if (!mbar_wait(&full[s], (it / S) & 1, g.status)) {
+      // warp-uniform: the MMAs are issued by one lane of a converged warp
+      if (!__all_sync(0xffffffffu, !*fail && mbar_wait(&full[s], (it / S) & 1, g.status))) {
         *fail = 1;
         break;
       }
@@ -127,12 +129,12 @@ __global__ void __launch_bounds__(128) nn_wgrad_kernel(const __grid_constant__ C
       for (int t = 0; t < TAPS; ++t)
 #pragma unroll
         for (int kk = 0; kk < WG_PX / 16; ++kk)
-          mma_bf16(tmem + t * BN, da + (uint64_t)(((kx0 + t) * 128 + kk * 2048) >> 4),
+          mma_bf16(el, tmem + t * BN, da + (uint64_t)(((kx0 + t) * 128 + kk * 2048) >> 4),
                    db + (uint64_t)((kk * 16 * Lay::RB) >> 4), idesc, (k > k0 || kk > 0) ? 1u : 0u);
-      mma_commit(&empty[s]);
+      mma_commit(el, &empty[s]);
     }
-    s_consumed = it;
-    mma_commit(acc);  // completes once every MMA issued above has finished
+    if (lane == 0) s_consumed = it;
+    mma_commit(el, acc);  // completes once every MMA issued above has finished
   }
   __syncthreads();
   const bool done = __all_sync(0xffffffffu, mbar_wait(acc, 0, g.status));
