@@ -12,7 +12,7 @@
 // function of the address.  Accumulation order as in nn_gemm_kernel (tap,
 // channel chunk, 16 channels), so the sums are the same.
 //
-//   warp 0 lane 0 -- TMA producer; warp 1 lane 0 -- MMA issuer into accumulator
+//   warp 0 -- TMA producer; warp 1 -- MMA issuer into accumulator
 //   (tile & 1); warps 2..5 -- epilogue of the finished accumulator.
 // Every wait is bounded; on a timeout the CTA records it, drains what it issued
 // and frees its TMEM.
@@ -90,25 +90,32 @@ __global__ void __launch_bounds__(192) nn_conv_row_kernel(const __grid_constant_
   const long long ntiles = (long long)g.N * g.tiles_x * g.H;
   const int t0 = (int)(ntiles * blockIdx.x / gridDim.x), t1 = (int)(ntiles * (blockIdx.x + 1) / gridDim.x);
 
-  if (warp == 0 && lane == 0) {
-    mbar_arrive_expect_tx(wfull, w_bytes);
-    for (int tap = 0; tap < 9; ++tap)
-      for (int c = 0; c < g.nchunk; ++c)
-        tma_load_3d(base + (tap * g.nchunk + c) * Lay::W_PANEL, &tmW, c * (RB / 2), tap, 0, wfull);
+  if (warp == 0) {  // all lanes run the loop, one issues
+    const uint32_t el = elect_one();
+    if (el) {
+      mbar_arrive_expect_tx(wfull, w_bytes);
+      for (int tap = 0; tap < 9; ++tap)
+        for (int c = 0; c < g.nchunk; ++c)
+          tma_load_3d(base + (tap * g.nchunk + c) * Lay::W_PANEL, &tmW, c * (RB / 2), tap, 0, wfull);
+    }
     int r = 0;  // rows loaded
-    for (int t = t0; t < t1 && !*fail; ++t) {
+    bool ok = true;
+    for (int t = t0; t < t1 && ok; ++t) {
       const int y = t % g.H, st = t / g.H;
       const int x = (st % g.tiles_x) * 128 - 1, n = st / g.tiles_x;
       for (int yy = (t == t0 || y == 0) ? y - 1 : y + 1; yy <= y + 1; ++yy, ++r) {
         const int s = r % R;
-        if (r >= R && !mbar_wait(&empty[s], ((r / R) - 1) & 1, g.status)) *fail = 1;
-        if (*fail) break;
-        mbar_arrive_expect_tx(&full[s], g.nchunk * 130 * RB);
-        for (int c = 0; c < g.nchunk; ++c)
-          tma_load_4d(rows + s * slot_bytes + c * Lay::PANEL, &tmX, c * (RB / 2), x, yy, n, &full[s]);
+        ok = __all_sync(0xffffffffu, !*fail && (r < R || mbar_wait(&empty[s], ((r / R) - 1) & 1, g.status)));
+        if (!ok) break;
+        if (el) {
+          mbar_arrive_expect_tx(&full[s], g.nchunk * 130 * RB);
+          for (int c = 0; c < g.nchunk; ++c)
+            tma_load_4d(rows + s * slot_bytes + c * Lay::PANEL, &tmX, c * (RB / 2), x, yy, n, &full[s]);
+        }
       }
     }
-    s_issued = r;
+    if (!ok) *fail = 1;
+    if (lane == 0) s_issued = r;
   } else if (warp == 1) {
     const uint32_t el = elect_one();
     const uint32_t idesc = mma_idesc_bf16(128, BN);

@@ -3,7 +3,7 @@
 //
 // One CTA computes a 128 x BN tile of D = sum_k A[m, k] B[n, k] (both
 // operands K-major) with the accumulator in tensor memory:
-//   warp 0 lane 0  -- TMA producer: per K step one A box (128 rows x RB
+//   warp 0         -- TMA producer (one elected lane): per K step one A box (128 rows x RB
 //                     bytes) and one B box (BN rows x RB bytes) into a stage
 //                     of an S-deep ring, 128/64-byte swizzled;
 //   warp 1         -- MMA issuer (one elected lane): RB/32 tcgen05.mma (K = 16) per stage, then
@@ -80,7 +80,7 @@ __device__ __forceinline__ GemmTile decode_tile(const GemmArgs& g, int t) {
 
 // Persistent CTA of 192 threads walking the tiles t = blockIdx.x,
 // blockIdx.x + gridDim.x, ...:
-//   warp 0 lane 0  -- TMA producer: per K step one A box (128 rows x RB
+//   warp 0         -- TMA producer (one elected lane): per K step one A box (128 rows x RB
 //                     bytes) and one B box (BN rows x RB bytes) into the next
 //                     stage of an S-deep ring that runs on across tiles;
 //   warp 1         -- MMA issuer (one elected lane): RB/32 tcgen05.mma (K = 16) per stage into
@@ -138,42 +138,54 @@ __global__ void __launch_bounds__(192, 1) nn_gemm_kernel(const __grid_constant__
   const uint32_t tmem = *tmem_slot;
   volatile int* fail = &s_fail;
 
-  if (warp == 0 && lane == 0) {
-    // ---- TMA producer
+  if (warp == 0) {
+    // ---- TMA producer (all lanes run the loop, one issues: coordinates and
+    // addresses stay in uniform registers)
+    const uint32_t el = elect_one();
     int it = 0;  // K steps issued, over all tiles of this CTA
-    for (int t = blockIdx.x; t < ntiles && !*fail; t += gridDim.x) {
+    bool ok = true;
+    for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
       const GemmTile q = decode_tile<BN>(g, t);
       const CUtensorMap* tmB = &tmB0;
       if (g.mode == MODE_WGRAD) {
         const int kx = q.tap % 3;
         tmB = kx == 0 ? &tmB0 : (kx == 1 ? &tmB1 : &tmB2);
       }
+      int tp = 0, chunk = 0;  // CONV: tap and channel chunk of the step
       for (int k = q.kbeg; k < q.kend; ++k) {
         const int s = it % S;
-        if (it >= S && !mbar_wait(&empty[s], ((it / S) - 1) & 1, g.status)) {
+        ok = __all_sync(0xffffffffu, !*fail && (it < S || mbar_wait(&empty[s], ((it / S) - 1) & 1, g.status)));
+        if (!ok) {
           *fail = 1;
           break;
         }
-        if (*fail) break;
         unsigned char* sa = base + s * Lay::STAGE;
         unsigned char* sb = sa + Lay::A_BYTES;
-        mbar_arrive_expect_tx(&full[s], Lay::STAGE);
         if (g.mode == MODE_CONV) {
-          const int tp = k / g.nchunk, c0 = (k % g.nchunk) * (RB / 2);
-          const int ky = tp / 3, kx = tp % 3;
-          tma_load_4d(sa, &tmA, c0, q.x0 - 1 + kx, q.y0 - 1 + ky, q.n_img, &full[s]);
-          tma_load_3d(sb, tmB, c0, tp, q.n0, &full[s]);
+          const int c0 = chunk * (RB / 2), ky = tp / 3, kx = tp - 3 * ky;
+          if (el) {
+            mbar_arrive_expect_tx(&full[s], Lay::STAGE);
+            tma_load_4d(sa, &tmA, c0, q.x0 - 1 + kx, q.y0 - 1 + ky, q.n_img, &full[s]);
+            tma_load_3d(sb, tmB, c0, tp, q.n0, &full[s]);
+          }
+          if (++chunk == g.nchunk) {
+            chunk = 0;
+            ++tp;
+          }
         } else {
           const int xc = k % g.wchunks, rest = k / g.wchunks;
           const int y = rest % g.H, n = rest / g.H;
           const int ky = q.tap / 3;
-          tma_load_4d(sa, &tmA, xc * 64, y, q.m0, n, &full[s]);
-          tma_load_4d(sb, tmB, xc * 64, y - 1 + ky, q.n0, n, &full[s]);
+          if (el) {
+            mbar_arrive_expect_tx(&full[s], Lay::STAGE);
+            tma_load_4d(sa, &tmA, xc * 64, y, q.m0, n, &full[s]);
+            tma_load_4d(sb, tmB, xc * 64, y - 1 + ky, q.n0, n, &full[s]);
+          }
         }
         ++it;
       }
     }
-    s_issued = it;
+    if (lane == 0) s_issued = it;
   } else if (warp == 1) {
     // ---- MMA issuer
     const uint32_t el = elect_one();

@@ -83,42 +83,66 @@ __global__ void to_chw_kernel(int n, int h, int w, int c, int cstride, int coff,
 }
 
 // Input convolution: 2 fp32 channels [n][2][h][w] -> c bf16 channels (ReLU).
+// A thread computes CIN_PX adjacent pixels of a row, so that a weight read from
+// shared memory (where it fits, as a broadcast of the whole block) serves that
+// many multiply-adds; with one pixel per thread the kernel was bound by those
+// reads (53 us for 32 channels of 8 x 256 x 512 pixels).
+constexpr int CIN_PX = 4;
 template <bool SMEM_W>
-__global__ void conv_in_fwd_kernel(int n, int h, int w, int c, const float* in, const float* W, const float* b,
-                                   bf16* out, int cstride, int coff) {
-  // the weights (18 per output channel) and biases: staged once per block
-  // where they fit, read by every thread of the block as broadcasts
-  extern __shared__ float cin_w[];
+__global__ void __launch_bounds__(128) conv_in_fwd_kernel(int n, int h, int w, int c, const float* in, const float* W,
+                                                          const float* b, bf16* out, int cstride, int coff) {
+  // weights of 8 output channels side by side: [c / 8][18 taps + bias][8]
+  extern __shared__ __align__(16) float cin_w[];
   if (SMEM_W) {
-    for (int k = threadIdx.x; k < 19 * c; k += blockDim.x) cin_w[k] = k < 18 * c ? W[k] : b[k - 18 * c];
+    for (int k = threadIdx.x; k < 19 * c; k += blockDim.x) {
+      const int co = k / 19, t = k - 19 * co;
+      cin_w[(co / 8 * 19 + t) * 8 + co % 8] = t < 18 ? W[co * 18 + t] : b[co];
+    }
     __syncthreads();
   }
-  const float* Wp = SMEM_W ? cin_w : W;
-  const float* bp = SMEM_W ? cin_w + 18 * c : b;
-  const long long total = (long long)n * h * w;
+  const int wq = (w + CIN_PX - 1) / CIN_PX;
+  const long long total = (long long)n * h * wq;
   GRID_STRIDE(i, total) {
-    const int x = (int)(i % w);
-    const int y = (int)((i / w) % h);
-    const int bb = (int)(i / ((long long)w * h));
-    float v[18];
-    for (int ci = 0; ci < 2; ++ci)
-      for (int ky = 0; ky < 3; ++ky)
-        for (int kx = 0; kx < 3; ++kx) {
-          const int yy = y - 1 + ky, xx = x - 1 + kx;
-          v[ci * 9 + ky * 3 + kx] =
-              (yy >= 0 && yy < h && xx >= 0 && xx < w) ? in[(((long long)bb * 2 + ci) * h + yy) * w + xx] : 0.f;
-        }
-    for (int c8 = 0; c8 < c; c8 += 8) {
-      float o[8];
+    const int x = (int)(i % wq) * CIN_PX;
+    const int y = (int)((i / wq) % h);
+    const int bb = (int)(i / ((long long)wq * h));
+    float v[6][CIN_PX + 2];  // [channel, ky][x - 1 ..]
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int co = c8 + j;
-        float a = bp[co];
+    for (int r = 0; r < 6; ++r) {
+      const int yy = y - 1 + r % 3;
+      const float* p = in + (((long long)bb * 2 + r / 3) * h + yy) * w;
 #pragma unroll
-        for (int k = 0; k < 18; ++k) a = fmaf(Wp[co * 18 + k], v[k], a);
-        o[j] = a > 0.f ? a : 0.f;
+      for (int k = 0; k < CIN_PX + 2; ++k) {
+        const int xx = x - 1 + k;
+        v[r][k] = (yy >= 0 && yy < h && xx >= 0 && xx < w) ? p[xx] : 0.f;
       }
-      st8(out + i * cstride + coff + c8, pack8(o));
+    }
+    bf16* o = out + (((long long)bb * h + y) * w + x) * cstride + coff;
+    for (int c8 = 0; c8 < c; c8 += 8) {
+      float a[CIN_PX][8];
+#pragma unroll
+      for (int t = -1; t < 18; ++t) {  // the bias, then the taps
+        float wt[8];
+        if (SMEM_W) {
+          const float4* q = reinterpret_cast<const float4*>(cin_w + (c8 / 8 * 19 + (t < 0 ? 18 : t)) * 8);
+          const float4 q0 = q[0], q1 = q[1];
+          wt[0] = q0.x; wt[1] = q0.y; wt[2] = q0.z; wt[3] = q0.w;
+          wt[4] = q1.x; wt[5] = q1.y; wt[6] = q1.z; wt[7] = q1.w;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) wt[j] = t < 0 ? __ldg(b + c8 + j) : __ldg(W + (c8 + j) * 18 + t);
+        }
+#pragma unroll
+        for (int k = 0; k < CIN_PX; ++k)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) a[k][j] = t < 0 ? wt[j] : fmaf(wt[j], v[(t < 0 ? 0 : t) / 3][k + (t < 0 ? 0 : t) % 3], a[k][j]);
+      }
+#pragma unroll
+      for (int k = 0; k < CIN_PX; ++k) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[k][j] = a[k][j] > 0.f ? a[k][j] : 0.f;
+        if (x + k < w) st8(o + (long long)k * cstride + c8, pack8(a[k]));
+      }
     }
   }
 }
@@ -148,31 +172,31 @@ __global__ void conv_out_fwd_kernel(int n, int h, int w, int c, const bf16* in, 
   }
 }
 
-// The same convolution for c <= 64 from shared memory: a block of 256
-// threads takes 256 pixels of one image row, stages the three input rows
-// (258 pixels with the halo, c channels, 16-byte vectors) and the weights
-// (tap-major) once, and each thread sums its pixel's 9 taps from there.  A
-// thread walks its pixel's channel vectors starting at (lane mod c/8), so
-// that the 8 threads of a 16-byte access phase hit distinct banks.
-constexpr int COUT_TX = 256;
+// The same convolution for 32 or 64 channels from shared memory: a block of
+// COUT_TX threads takes COUT_TX columns of COUT_R rows, stages the COUT_R + 2
+// input rows (with the column halo, c channels, 16-byte vectors) and the
+// weights (tap-major) once, and each thread sums its column's COUT_R pixels,
+// each weight read serving all of them.  A thread walks a pixel's channel
+// vectors starting at (lane mod c/8), so that the 8 threads of a 16-byte access
+// phase hit distinct banks.  One row per block staged every row three times
+// and read the weights once per pixel: 80 us for 32 channels of 8 x 256 x 512.
+constexpr int COUT_TX = 128, COUT_R = 4;
 template <int CV>  // channel vectors per pixel (c = 8 CV)
 __global__ void __launch_bounds__(COUT_TX) conv_out_tile_kernel(int n, int h, int w, const bf16* in, int cstride,
                                                                  const float* W, const float* b, float* out) {
   extern __shared__ __align__(16) unsigned char cout_smem[];
-  constexpr int cv = CV, c = 8 * CV, cols = COUT_TX + 2;
-  uint4* srow = reinterpret_cast<uint4*>(cout_smem);  // [3][cols][cv]
-  float* ws = reinterpret_cast<float*>(srow + 3 * cols * cv);  // [9][c]
-  const int ntx = (w + COUT_TX - 1) / COUT_TX;
-  const int xt = blockIdx.x % ntx;
-  const long long ry = blockIdx.x / ntx;
-  const int y = (int)(ry % h), bb = (int)(ry / h);
-  const int x0 = xt * COUT_TX;
+  constexpr int cv = CV, c = 8 * CV, cols = COUT_TX + 2, rows = COUT_R + 2;
+  uint4* srow = reinterpret_cast<uint4*>(cout_smem);  // [rows][cols][cv]
+  float* ws = reinterpret_cast<float*>(srow + rows * cols * cv);  // [9][c]
+  const int ntx = (w + COUT_TX - 1) / COUT_TX, nty = (h + COUT_R - 1) / COUT_R;
+  const int x0 = (blockIdx.x % ntx) * COUT_TX;
+  const int y0 = (blockIdx.x / ntx % nty) * COUT_R, bb = blockIdx.x / (ntx * nty);
   for (int k = threadIdx.x; k < 9 * c; k += COUT_TX) {
     const int tap = k / c, ci = k - tap * c;
     ws[k] = W[ci * 9 + tap];
   }
   // eight vectors per thread in flight at a time: loads first, then stores
-  const int nvec = 3 * cols * cv;
+  constexpr int nvec = rows * cols * cv;
   for (int k0 = threadIdx.x; k0 < nvec; k0 += 8 * COUT_TX) {
     uint4 q[8];
 #pragma unroll
@@ -182,7 +206,7 @@ __global__ void __launch_bounds__(COUT_TX) conv_out_tile_kernel(int n, int h, in
       if (k < nvec) {
         const int v = k % cv, rc = k / cv;
         const int col = rc % cols, r = rc / cols;
-        const int yy = y - 1 + r, xx = x0 - 1 + col;
+        const int yy = y0 - 1 + r, xx = x0 - 1 + col;
         if (yy >= 0 && yy < h && xx >= 0 && xx < w) q[u] = ld8(in + (((long long)bb * h + yy) * w + xx) * cstride + 8 * v);
       }
     }
@@ -193,8 +217,13 @@ __global__ void __launch_bounds__(COUT_TX) conv_out_tile_kernel(int n, int h, in
   __syncthreads();
   const int t = threadIdx.x, x = x0 + t;
   if (x >= w) return;
-  float acc[4] = {b[0], 0.f, 0.f, 0.f};  // four partial sums: short FMA chains
+  float acc[COUT_R][4];  // four partial sums per pixel: short FMA chains
 #pragma unroll
+  for (int i = 0; i < COUT_R; ++i) {
+    acc[i][0] = b[0];
+    acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+  }
+#pragma unroll 3
   for (int tap = 0; tap < 9; ++tap) {
     const int ky = tap / 3, kx = tap - 3 * ky;
     const uint4* px = srow + (ky * cols + t + kx) * cv;
@@ -202,41 +231,77 @@ __global__ void __launch_bounds__(COUT_TX) conv_out_tile_kernel(int n, int h, in
 #pragma unroll
     for (int vv = 0; vv < cv; ++vv) {
       const int v = (vv + t) & (cv - 1);
-      float f[8];
-      unpack8(px[v], f);
+      const float4 w0 = lds4(wt + 8 * v), w1 = lds4(wt + 8 * v + 4);
+      const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j & 3] = fmaf(wt[8 * v + j], f[j], acc[j & 3]);
+      for (int i = 0; i < COUT_R; ++i) {
+        float f[8];
+        unpack8(px[i * cols * cv + v], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j & 3] = fmaf(wv[j], f[j], acc[i][j & 3]);
+      }
     }
   }
-  out[((long long)bb * h + y) * w + x] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+#pragma unroll
+  for (int i = 0; i < COUT_R; ++i)
+    if (y0 + i < h) out[((long long)bb * h + y0 + i) * w + x] = (acc[i][0] + acc[i][1]) + (acc[i][2] + acc[i][3]);
 }
 
 // Data gradient of the output convolution, times [act > 0] (the ReLU of the
 // layer that produced its input): dx[p][ci] = sum_tap W[ci][tap] g[p - off].
-__global__ void conv_out_dgrad_kernel(int n, int h, int w, int c, const float* g, const float* W, const bf16* act,
-                                      int act_cstride, bf16* dx) {
-  const long long total = (long long)n * h * w;
+// A thread takes one channel vector of COD_PX adjacent pixels of a row, so that
+// the 72 weights it reads (shared memory, tap-major) serve all of them; with
+// the weights read from global memory for every pixel it took 60 us for 32
+// channels of 8 x 256 x 512.
+constexpr int COD_PX = 4;
+__global__ void __launch_bounds__(256) conv_out_dgrad_kernel(int n, int h, int w, int c, const float* g, const float* W,
+                                                             const bf16* act, int act_cstride, bf16* dx) {
+  extern __shared__ __align__(16) float cod_w[];  // [9][c]
+  for (int k = threadIdx.x; k < 9 * c; k += blockDim.x) cod_w[k] = W[(k % c) * 9 + k / c];
+  __syncthreads();
+  const int cv = c / 8, wq = (w + COD_PX - 1) / COD_PX;
+  const long long total = (long long)n * h * wq * cv;
   GRID_STRIDE(i, total) {
-    const int x = (int)(i % w);
-    const int y = (int)((i / w) % h);
-    const int bb = (int)(i / ((long long)w * h));
-    float gv[9];
-    for (int ky = 0; ky < 3; ++ky)
-      for (int kx = 0; kx < 3; ++kx) {
-        // output pixel (y + 1 - ky, x + 1 - kx) reads this pixel through tap (ky, kx)
-        const int yy = y + 1 - ky, xx = x + 1 - kx;
-        gv[ky * 3 + kx] = (yy >= 0 && yy < h && xx >= 0 && xx < w) ? g[((long long)bb * h + yy) * w + xx] : 0.f;
-      }
-    for (int c8 = 0; c8 < c; c8 += 8) {
-      float o[8], m[8];
-      unpack8(ld8(act + i * act_cstride + c8), m);
+    const int c8 = (int)(i % cv) * 8;
+    const long long q = i / cv;
+    const int x = (int)(q % wq) * COD_PX;
+    const int y = (int)((q / wq) % h);
+    const int bb = (int)(q / ((long long)wq * h));
+    float gv[3][COD_PX + 2];  // rows y + 1, y, y - 1; columns x - 1 ..
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float a = 0.f;
-        for (int k = 0; k < 9; ++k) a = fmaf(W[(c8 + j) * 9 + k], gv[k], a);
-        o[j] = m[j] > 0.f ? a : 0.f;
+    for (int r = 0; r < 3; ++r) {
+      const int yy = y + 1 - r;
+      const float* p = g + ((long long)bb * h + yy) * w;
+#pragma unroll
+      for (int k = 0; k < COD_PX + 2; ++k) {
+        const int xx = x - 1 + k;
+        gv[r][k] = (yy >= 0 && yy < h && xx >= 0 && xx < w) ? p[xx] : 0.f;
       }
-      st8(dx + i * c + c8, pack8(o));
+    }
+    float o[COD_PX][8];
+#pragma unroll
+    for (int k = 0; k < COD_PX; ++k)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[k][j] = 0.f;
+#pragma unroll
+    for (int t = 0; t < 9; ++t) {
+      // output pixel (y + 1 - ky, x + 1 - kx) reads this pixel through tap (ky, kx)
+      const float4 w0 = lds4(cod_w + t * c + c8), w1 = lds4(cod_w + t * c + c8 + 4);
+      const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+      for (int k = 0; k < COD_PX; ++k)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[k][j] = fmaf(wv[j], gv[t / 3][k + 2 - t % 3], o[k][j]);
+    }
+    const long long pix = ((long long)bb * h + y) * w + x;
+#pragma unroll
+    for (int k = 0; k < COD_PX; ++k) {
+      if (x + k >= w) break;
+      float m[8];
+      unpack8(ld8(act + (pix + k) * act_cstride + c8), m);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[k][j] = m[j] > 0.f ? o[k][j] : 0.f;
+      st8(dx + (pix + k) * c + c8, pack8(o[k]));
     }
   }
 }
@@ -246,99 +311,115 @@ __global__ void conv_out_dgrad_kernel(int n, int h, int w, int c, const float* g
 // v a bf16 NHWC tensor (channel vectors of 8), s an fp32 image (0 outside).
 // Input convolution: v = dy, s = an input channel, d_k = (ky - 1, kx - 1);
 // output convolution: v = the layer's input, s = dy, d_k = (1 - ky, 1 - kx).
-// A thread owns one column and 8 channels, walks VS_ROWS rows with the 3 x 3
-// window of s in registers and keeps the 72 sums of its channels; each v
-// vector is read once.  One block per channel with scalar reads at the pixel
-// stride took 553 us (output) and 398 us (input) for 32 channels of 8 x 256 x
-// 512 pixels.
-constexpr int VS_ROWS = 16, VS_CG = 4, VS_X = 64;  // rows, channel vectors, columns per block
-// VEC: the vectors are 16-byte aligned and whole; else channel by channel.
-template <int SIGN, bool VEC>
-__global__ void __launch_bounds__(VS_CG* VS_X) vec_scalar_wgrad_kernel(int h, int w, int c, const bf16* v, int v_cstride,
-                                                                       const float* s, long long s_image,
-                                                                       float* dW, int w_stride, float* db_vec,
-                                                                       float* db_scalar) {
-  __shared__ float red[VS_CG * VS_X / 32][VS_CG][8];
-  const int cg = threadIdx.x % VS_CG, cv = blockIdx.y * VS_CG + cg;
+// A thread owns one column and VS_C = 8 / NI channels, walks VS_ROWS rows with
+// the 3 x 3 windows of the NI images in registers and keeps the 72 sums of its
+// channels; each v vector is read once.  One block per channel with scalar reads
+// at the pixel stride took 553 us (output) and 398 us (input) for 32 channels of
+// 8 x 256 x 512 pixels; 16 rows per block, whose 80 sums per thread then meet
+// through shuffles, 99 us (output) and 2 x 74 us (input, one image at a time).
+constexpr int VS_ROWS = 64, VS_X = 64;  // rows and columns per block
+template <int SIGN, int NI, bool VEC>
+__global__ void __launch_bounds__(256) vec_scalar_wgrad_kernel(int h, int w, int c, const bf16* v, int v_cstride,
+                                                               const float* s, float* dW, float* db_vec,
+                                                               float* db_scalar) {
+  constexpr int VS_C = 8 / NI, CG = 256 / VS_X;  // channels per thread, channel groups per block
+  // the block's part of the images with its halo (0 outside); then the warps' sums
+  constexpr int TW = VS_X + 2, TILE = NI * (VS_ROWS + 2) * TW, RED = 8 * CG * (9 * NI + 1) * VS_C;
+  __shared__ float sm[TILE > RED ? TILE : RED];
+  const int cg = threadIdx.x % CG, c0 = (blockIdx.y * CG + cg) * VS_C;
   const int ntx = (w + VS_X - 1) / VS_X, nty = (h + VS_ROWS - 1) / VS_ROWS;
-  const int x = (blockIdx.x % ntx) * VS_X + threadIdx.x / VS_CG;
+  const int x = (blockIdx.x % ntx) * VS_X + threadIdx.x / CG;
   const int y0 = (blockIdx.x / ntx % nty) * VS_ROWS, n = blockIdx.x / (ntx * nty);
-  const bool in = x < w && cv * 8 < c;
-  const float* img = s + n * s_image;
-  const bf16* vp = v + ((long long)n * h + y0) * w * v_cstride + (long long)x * v_cstride + cv * 8;
-  auto row = [&](int y, float (&r)[3]) {
+  const bool in = x < w && c0 < c;
+  const long long hw = (long long)h * w;
+  const float* img = s + n * NI * hw;
+  const bf16* vp = v + ((long long)n * h + y0) * w * v_cstride + (long long)x * v_cstride + c0;
+  float acc[NI][9][VS_C], bias[VS_C], sc = 0.f;
+  auto vec = [&](int r, float (&f)[VS_C]) {  // 0 beyond the image or the channels
+    const bf16* q = vp + (long long)r * w * v_cstride;
+    const bool ok = in && y0 + r < h;
+    if constexpr (!VEC) {
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const int xx = x + d - 1;
-      r[d] = (y >= 0 && y < h && xx >= 0 && xx < w) ? __ldg(img + (long long)y * w + xx) : 0.f;
+      for (int j = 0; j < VS_C; ++j) f[j] = ok && c0 + j < c ? ld(q + j) : 0.f;
+    } else if constexpr (VS_C == 8) {
+      unpack8(ok ? ld8(q) : make_uint4(0u, 0u, 0u, 0u), f);
+    } else {
+      const uint2 u = ok ? __ldg(reinterpret_cast<const uint2*>(q)) : make_uint2(0u, 0u);
+      f[0] = __uint_as_float(u.x << 16);
+      f[1] = __uint_as_float(u.x & 0xffff0000u);
+      f[2] = __uint_as_float(u.y << 16);
+      f[3] = __uint_as_float(u.y & 0xffff0000u);
     }
   };
-  float acc[9][8], bias[8], sc = 0.f;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
+  for (int j = 0; j < VS_C; ++j) {
     bias[j] = 0.f;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) acc[k][j] = 0.f;
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+      for (int k = 0; k < 9; ++k) acc[i][k][j] = 0.f;
   }
-  float win[3][3];
-  row(y0 - 1, win[0]);
-  row(y0, win[1]);
-#pragma unroll 4
-  for (int i = 0; i < VS_ROWS; ++i) {
-    const int y = y0 + i;
-    row(y + 1, win[2]);
-    if (in && y < h) {
-      float f[8];
-      const bf16* q = vp + (long long)i * w * v_cstride;
-      if constexpr (VEC) {
-        unpack8(ld8(q), f);
-      } else {
+  for (int q = threadIdx.x; q < TILE; q += 256) {
+    const int i = q / ((VS_ROWS + 2) * TW), rr = q / TW % (VS_ROWS + 2), cc = q % TW;
+    const int yy = y0 - 1 + rr, xx = blockIdx.x % ntx * VS_X - 1 + cc;
+    sm[q] = (yy >= 0 && yy < h && xx >= 0 && xx < w) ? __ldg(img + i * hw + (long long)yy * w + xx) : 0.f;
+  }
+  __syncthreads();
+  const float* tile = sm + threadIdx.x / CG;
+  // four rows' vector loads are issued together
+#pragma unroll 1
+  for (int r0 = 0; r0 < VS_ROWS && y0 + r0 < h; r0 += 4) {
+    float f[4][VS_C], win[NI][6][3];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) f[j] = cv * 8 + j < c ? ld(q + j) : 0.f;
+    for (int r = 0; r < 4; ++r) vec(r0 + r, f[r]);
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+      for (int q = 0; q < 6; ++q)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) win[i][q][d] = tile[(i * (VS_ROWS + 2) + r0 + q) * TW + d];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      if (in && y0 + r0 + r < h) sc += win[0][r + 1][1];
+#pragma unroll
+      for (int j = 0; j < VS_C; ++j) {
+        bias[j] += f[r][j];
+#pragma unroll
+        for (int i = 0; i < NI; ++i)
+#pragma unroll
+          for (int k = 0; k < 9; ++k) {
+            const int t = SIGN > 0 ? k : 8 - k;
+            acc[i][k][j] = fmaf(f[r][j], win[i][r + t / 3][t % 3], acc[i][k][j]);
+          }
       }
-      sc += win[1][1];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        bias[j] += f[j];
-#pragma unroll
-        for (int k = 0; k < 9; ++k) {
-          const int t = SIGN > 0 ? k : 8 - k;
-          acc[k][j] = fmaf(f[j], win[t / 3][t % 3], acc[k][j]);
-        }
-      }
-    }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      win[0][d] = win[1][d];
-      win[1][d] = win[2][d];
     }
   }
   // lanes of equal cg, then the block's warps, then one addition per sum
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  constexpr int NWARP = VS_CG * VS_X / 32;
+  __syncthreads();
+  auto red = [&](int u, int g, int k, int j) -> float& { return sm[((u * CG + g) * (9 * NI + 1) + k) * VS_C + j]; };
 #pragma unroll
-  for (int k = 0; k < 10; ++k) {
+  for (int k = 0; k <= 9 * NI; ++k)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float a = k < 9 ? acc[k < 9 ? k : 0][j] : bias[j];
+    for (int j = 0; j < VS_C; ++j) {
+      float a = k < 9 * NI ? acc[k / 9 < NI ? k / 9 : 0][k % 9][j] : bias[j];
 #pragma unroll
-      for (int o = 16; o >= VS_CG; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-      if (lane < VS_CG) red[wid][lane][j] = a;
+      for (int o = 16; o >= CG; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      if (lane < CG) red(wid, lane, k, j) = a;
     }
-    __syncthreads();
-    if (threadIdx.x < VS_CG * 8) {
-      const int g = threadIdx.x / 8, j = threadIdx.x % 8, ch = (blockIdx.y * VS_CG + g) * 8 + j;
-      float a = 0.f;
+  __syncthreads();
+  for (int q = threadIdx.x; q < CG * (9 * NI + 1) * VS_C; q += 256) {
+    const int j = q % VS_C, k = q / VS_C % (9 * NI + 1), g = q / (VS_C * (9 * NI + 1));
+    const int ch = (blockIdx.y * CG + g) * VS_C + j;
+    float a = 0.f;
 #pragma unroll
-      for (int q = 0; q < NWARP; ++q) a += red[q][g][j];
-      if (ch < c) {
-        if (k < 9)
-          atomicAdd(dW + (long long)ch * w_stride + k, a);
-        else if (db_vec != nullptr)
-          atomicAdd(db_vec + ch, a);
-      }
+    for (int u = 0; u < 8; ++u) a += red(u, g, k, j);
+    if (ch < c) {
+      if (k < 9 * NI)
+        atomicAdd(dW + (long long)ch * 9 * NI + k, a);
+      else if (db_vec != nullptr)
+        atomicAdd(db_vec + ch, a);
     }
-    __syncthreads();
   }
   if (db_scalar != nullptr && blockIdx.y == 0) {
     if (cg != 0) sc = 0.f;
@@ -482,7 +563,7 @@ __global__ void __launch_bounds__(256) bias_grad_nhwc_kernel(long long pixels, i
   __syncthreads();
   float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (p0 < per) {
-#pragma unroll 4
+#pragma unroll 8
     for (long long p = (long long)blockIdx.x * per + p0; p < pixels; p += (long long)gridDim.x * per) {
       float f[8];
       unpack8(ld8(dy + p * c + 8 * v), f);
@@ -559,12 +640,12 @@ cudaError_t launch_to_chw(int n, int h, int w, int c, int cstride, int coff, con
 
 cudaError_t launch_conv_in_fwd(int n, int h, int w, int c, const float* in, const float* W, const float* b, bf16* out,
                                int cstride, int coff, cudaStream_t s) {
+  const long long threads = (long long)n * h * ((w + CIN_PX - 1) / CIN_PX);
+  const int blocks = blocks_for(2 * threads);
   if (c <= 256)
-    conv_in_fwd_kernel<true><<<blocks_for((long long)n * h * w), 256, (size_t)19 * c * 4, s>>>(n, h, w, c, in, W, b,
-                                                                                           out, cstride, coff);
+    conv_in_fwd_kernel<true><<<blocks, 128, (size_t)19 * c * 4, s>>>(n, h, w, c, in, W, b, out, cstride, coff);
   else
-    conv_in_fwd_kernel<false><<<blocks_for((long long)n * h * w), 256, 0, s>>>(n, h, w, c, in, W, b, out, cstride,
-                                                                              coff);
+    conv_in_fwd_kernel<false><<<blocks, 128, 0, s>>>(n, h, w, c, in, W, b, out, cstride, coff);
   return cudaGetLastError();
 }
 
@@ -574,20 +655,18 @@ static long long vs_blocks(int n, int h, int w) {
 
 cudaError_t launch_conv_in_wgrad(int n, int h, int w, int c, const float* in, const bf16* dy, int dy_cstride,
                                  float* dW, float* db, cudaStream_t s) {
-  const dim3 grid((unsigned)vs_blocks(n, h, w), (unsigned)(((c + 7) / 8 + VS_CG - 1) / VS_CG));
-  const long long hw = (long long)h * w;
-  const bool vec = c % 8 == 0 && dy_cstride % 8 == 0 && (reinterpret_cast<uintptr_t>(dy) & 15u) == 0;
-  auto kern = vec ? vec_scalar_wgrad_kernel<1, true> : vec_scalar_wgrad_kernel<1, false>;
-  for (int ci = 0; ci < 2; ++ci)
-    kern<<<grid, VS_CG * VS_X, 0, s>>>(h, w, c, dy, dy_cstride, in + ci * hw, 2 * hw, dW + 9 * ci, 18,
-                                       ci == 0 ? db : nullptr, nullptr);
+  // 4 channel groups of 4 channels per block
+  const dim3 grid((unsigned)vs_blocks(n, h, w), (unsigned)((c + 15) / 16));
+  const bool vec = c % 4 == 0 && dy_cstride % 4 == 0 && (reinterpret_cast<uintptr_t>(dy) & 7u) == 0;
+  auto kern = vec ? vec_scalar_wgrad_kernel<1, 2, true> : vec_scalar_wgrad_kernel<1, 2, false>;
+  kern<<<grid, 256, 0, s>>>(h, w, c, dy, dy_cstride, in, dW, db, nullptr);
   return cudaGetLastError();
 }
 
 cudaError_t launch_conv_out_fwd(int n, int h, int w, int c, const bf16* in, int cstride, const float* W,
                                 const float* b, float* out, cudaStream_t s) {
   if (c == 32 || c == 64) {
-    const size_t smem = (size_t)3 * (COUT_TX + 2) * (c / 8) * 16 + (size_t)9 * c * 4;
+    const size_t smem = (size_t)(COUT_R + 2) * (COUT_TX + 2) * (c / 8) * 16 + (size_t)9 * c * 4;
     auto kern = c == 32 ? conv_out_tile_kernel<4> : conv_out_tile_kernel<8>;
     static bool set[2] = {false, false};
     if (!set[c == 64]) {
@@ -595,7 +674,7 @@ cudaError_t launch_conv_out_fwd(int n, int h, int w, int c, const bf16* in, int 
       if (e != cudaSuccess) return e;
       set[c == 64] = true;
     }
-    const long long blocks = (long long)n * h * ((w + COUT_TX - 1) / COUT_TX);
+    const long long blocks = (long long)n * ((h + COUT_R - 1) / COUT_R) * ((w + COUT_TX - 1) / COUT_TX);
     kern<<<(unsigned)blocks, COUT_TX, smem, s>>>(n, h, w, in, cstride, W, b, out);
     return cudaGetLastError();
   }
@@ -605,10 +684,16 @@ cudaError_t launch_conv_out_fwd(int n, int h, int w, int c, const bf16* in, int 
 
 cudaError_t launch_conv_out_bwd(int n, int h, int w, int c, const float* g, const float* W, const bf16* act,
                                 int act_cstride, bf16* dx, float* dW, float* db, cudaStream_t s) {
-  conv_out_dgrad_kernel<<<blocks_for((long long)n * h * w), 256, 0, s>>>(n, h, w, c, g, W, act, act_cstride, dx);
-  const dim3 grid((unsigned)vs_blocks(n, h, w), (unsigned)((c / 8 + VS_CG - 1) / VS_CG));
-  vec_scalar_wgrad_kernel<-1, true><<<grid, VS_CG * VS_X, 0, s>>>(h, w, c, act, act_cstride, g, (long long)h * w, dW,
-                                                                   9, nullptr, db);
+  const size_t smem = (size_t)9 * c * sizeof(float);
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(conv_out_dgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  conv_out_dgrad_kernel<<<blocks_for((long long)n * h * ((w + COD_PX - 1) / COD_PX) * (c / 8)), 256, smem, s>>>(
+      n, h, w, c, g, W, act, act_cstride, dx);
+  // 4 channel groups of 8 channels per block
+  const dim3 grid((unsigned)vs_blocks(n, h, w), (unsigned)((c + 31) / 32));
+  vec_scalar_wgrad_kernel<-1, 1, true><<<grid, 256, 0, s>>>(h, w, c, act, act_cstride, g, dW, nullptr, db);
   return cudaGetLastError();
 }
 
@@ -647,7 +732,7 @@ cudaError_t launch_bias_grad(int n, long long hw, int c, const bf16* dy, float* 
 
 cudaError_t launch_bias_grad_nhwc(long long pixels, int c, const bf16* dy, float* db, cudaStream_t s) {
   if (c > 2048) return cudaErrorInvalidValue;  // one channel vector per thread
-  long long b = (pixels * (c / 8) + 256 * 16 - 1) / (256 * 16);
+  long long b = (pixels * (c / 8) + 256 * 32 - 1) / (256 * 32);
   b = b > 152 * 8 ? 152 * 8 : b;
   bias_grad_nhwc_kernel<<<(unsigned)b, 256, (size_t)c * 4, s>>>(pixels, c, dy, db);
   return cudaGetLastError();

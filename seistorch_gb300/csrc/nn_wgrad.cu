@@ -39,13 +39,15 @@ namespace {
 constexpr int WG_PX = 64;                  // pixels per K step
 constexpr int WG_A_ROWS = WG_PX + 2;       // with the halo of the kx taps
 constexpr int WG_A_PANEL = 9216;           // 66 rows of 128 bytes, to the next 1024
-template <int BN, int TAPS>
+template <int BN, int TAPS, bool ALONE>
 struct WgLayout {
   static constexpr int RB = BN >= 64 ? 128 : 64;  // bytes of a B row
   static constexpr int B_PANELS = BN >= 64 ? BN / 64 : 1;
   static constexpr int B_PANEL = WG_PX * RB;
   static constexpr int STAGE = 2 * WG_A_PANEL + B_PANELS * B_PANEL;
-  static constexpr int S = BN == 128 ? 5 : 4;
+  // stages: about 200 KB where a CTA has the SM alone (eight steps in flight:
+  // a step's copies take about two steps' time to arrive), half where two share it
+  static constexpr int S = BN == 128 ? 6 : (ALONE ? 8 : 4);
   static constexpr int BYTES = S * STAGE + 1024 + 256;
   static constexpr int COLS = TAPS == 1 ? BN : (BN == 128 ? 512 : (BN == 64 ? 256 : 128));  // TAPS BN, to a power of two
 };
@@ -56,10 +58,10 @@ __device__ __forceinline__ uint64_t mn_desc(uint32_t addr, uint32_t lbo, uint32_
          (layout << 61);
 }
 
-template <int BN, int TAPS>
+template <int BN, int TAPS, bool ALONE>
 __global__ void __launch_bounds__(128) nn_wgrad_kernel(const __grid_constant__ CUtensorMap tmX,
                                                        const __grid_constant__ CUtensorMap tmD, const WgradArgs g) {
-  using Lay = WgLayout<BN, TAPS>;
+  using Lay = WgLayout<BN, TAPS, ALONE>;
   constexpr int S = Lay::S;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -90,26 +92,35 @@ __global__ void __launch_bounds__(128) nn_wgrad_kernel(const __grid_constant__ C
   const int k0 = blockIdx.x * g.k_per_split, k1 = min(k0 + g.k_per_split, g.kiters);
   const int panels = g.Cin - m0 > 64 ? 2 : 1;  // rows beyond Cin: not loaded, their sums not stored
 
-  if (warp == 0 && lane == 0) {
-    int it = 0;
-    for (int k = k0; k < k1 && !*fail; ++k, ++it) {
+  if (warp == 0) {
+    const uint32_t el = elect_one();
+    int xc = k0 % g.wchunks, y = k0 / g.wchunks % g.H, n = k0 / g.wchunks / g.H, it = 0;
+    for (int k = k0; k < k1; ++k, ++it) {
       const int s = it % S;
-      if (it >= S && !mbar_wait(&empty[s], ((it / S) - 1) & 1, g.status)) {
+      // warp-uniform, one lane issues
+      if (!__all_sync(0xffffffffu, !*fail && (it < S || mbar_wait(&empty[s], ((it / S) - 1) & 1, g.status)))) {
         *fail = 1;
         break;
       }
-      if (*fail) break;
-      const int xc = k % g.wchunks, rest = k / g.wchunks;
-      const int y = rest % g.H, n = rest / g.H;
-      unsigned char* sa = base + s * Lay::STAGE;
-      unsigned char* sb = sa + 2 * WG_A_PANEL;
-      mbar_arrive_expect_tx(&full[s], panels * WG_A_ROWS * 128 + Lay::B_PANELS * Lay::B_PANEL);
-      for (int p = 0; p < panels; ++p)
-        tma_load_4d(sa + p * WG_A_PANEL, &tmX, m0 + 64 * p, xc * WG_PX - 1, y + ky - 1, n, &full[s]);
-      for (int p = 0; p < Lay::B_PANELS; ++p)
-        tma_load_4d(sb + p * Lay::B_PANEL, &tmD, n0 + 64 * p, xc * WG_PX, y, n, &full[s]);
+      if (el) {
+        unsigned char* sa = base + s * Lay::STAGE;
+        unsigned char* sb = sa + 2 * WG_A_PANEL;
+        mbar_arrive_expect_tx(&full[s], panels * WG_A_ROWS * 128 + Lay::B_PANELS * Lay::B_PANEL);
+        tma_load_4d(sa, &tmX, m0, xc * WG_PX - 1, y + ky - 1, n, &full[s]);
+        if (panels > 1) tma_load_4d(sa + WG_A_PANEL, &tmX, m0 + 64, xc * WG_PX - 1, y + ky - 1, n, &full[s]);
+#pragma unroll
+        for (int p = 0; p < Lay::B_PANELS; ++p)
+          tma_load_4d(sb + p * Lay::B_PANEL, &tmD, n0 + 64 * p, xc * WG_PX, y, n, &full[s]);
+      }
+      if (++xc == g.wchunks) {
+        xc = 0;
+        if (++y == g.H) {
+          y = 0;
+          ++n;
+        }
+      }
     }
-    s_issued = it;
+    if (lane == 0) s_issued = it;
   } else if (warp == 1) {
     const uint32_t el = elect_one();
     const uint32_t idesc = mma_idesc_bf16(128, BN) | (1u << 15) | (1u << 16);  // A and B MN-major
@@ -168,10 +179,17 @@ __global__ void __launch_bounds__(128) nn_wgrad_kernel(const __grid_constant__ C
   }
 }
 
-template <int BN, int TAPS>
-cudaError_t launch_t(const CUtensorMap* maps, const WgradArgs& g, int splits, cudaStream_t s) {
-  using Lay = WgLayout<BN, TAPS>;
-  auto kern = nn_wgrad_kernel<BN, TAPS>;
+int sm_count() {
+  int dev = 0, sms = 152;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+template <int BN, int TAPS, bool ALONE>
+cudaError_t launch_s(const CUtensorMap* maps, const WgradArgs& g, int splits, cudaStream_t s) {
+  using Lay = WgLayout<BN, TAPS, ALONE>;
+  auto kern = nn_wgrad_kernel<BN, TAPS, ALONE>;
   static bool set = false;
   if (!set) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay::BYTES);
@@ -179,28 +197,40 @@ cudaError_t launch_t(const CUtensorMap* maps, const WgradArgs& g, int splits, cu
     if (e != cudaSuccess) return e;
     set = true;
   }
-  // residency: two CTAs per SM (90 / 107 KB of stages; 128 / 256 of the 512
-  // TMEM columns), one for BN = 128
   const dim3 grid((unsigned)splits, (unsigned)(9 / TAPS * ((g.Cin + 127) / 128)), (unsigned)((g.Cout + BN - 1) / BN));
   kern<<<grid, 128, Lay::BYTES, s>>>(maps[0], maps[1], g);
   return cudaGetLastError();
 }
 
+template <int BN, int TAPS>
+cudaError_t launch_t(const CUtensorMap* maps, const WgradArgs& g, int splits, cudaStream_t s) {
+  const long long ctas = (long long)splits * (9 / TAPS) * ((g.Cin + 127) / 128) * ((g.Cout + BN - 1) / BN);
+  return ctas <= sm_count() ? launch_s<BN, TAPS, true>(maps, g, splits, s) : launch_s<BN, TAPS, false>(maps, g, splits, s);
+}
+
 }  // namespace
 
-// Output channels per tile and taps per CTA: the widest that still gives each
-// SM a CTA.  The B box of the tensor map is 64 channels (32 for bn = 32).
+// Output channels per tile and taps per CTA of least estimated time.  Cycles of
+// a step measured at the layers' sizes (batch 8 of 256 x 512): 62 / 78 per MMA
+// of 32 / 64 output channels, and about 600 where the copies' latency, not the
+// MMAs, is what a step waits for (one tap).  128 -> 128 channels: 64 us as three
+// taps by 64, 40 us as one tap by 64; 384 -> 128: 162 us as one tap by 128 in
+// two waves, 75 us as three taps by 64 in one.  The B box of the tensor map is
+// 64 channels (32 for bn = 32).
 static void wgrad_tile(const WgradArgs& g, int splits, int* bn, int* taps) {
-  int dev = 0, sms = 152;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  *bn = g.Cout >= 128 ? 128 : (g.Cout > 32 ? 64 : 32);
-  *taps = 3;
-  const int mt = (g.Cin + 127) / 128;
-  auto ctas = [&]() { return splits * (9 / *taps) * mt * ((g.Cout + *bn - 1) / *bn); };
-  if (ctas() < sms) *taps = 1;
-  if (ctas() < sms && *bn == 128) *bn = 64;
-  if (ctas() < sms && *bn == 64) *bn = 32;
+  const int sms = sm_count(), mt = (g.Cin + 127) / 128;
+  int best = 0;
+  for (int t : {3, 1})
+    for (int n : {128, 64, 32}) {
+      if (n > 32 && g.Cout <= n / 2) continue;  // half the tile empty
+      const int ctas = splits * (9 / t) * mt * ((g.Cout + n - 1) / n), mma = 4 * t * (46 + n / 2);
+      const int cost = (ctas + sms - 1) / sms * (mma > 600 ? mma : 600);
+      if (best == 0 || cost < best) {
+        best = cost;
+        *bn = n;
+        *taps = t;
+      }
+    }
 }
 
 static int wgrad_splits(const WgradArgs& g, int* per) {
