@@ -85,6 +85,9 @@ __global__ void __launch_bounds__(192) nn_conv_row_kernel(const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  // the barriers and the TMEM are set up beside the previous launch
+  pdl_wait();
+  pdl_trigger();
   volatile int* fail = &s_fail;
   // tiles in the order image, strip, row (rows fastest); this CTA's range
   const long long ntiles = (long long)g.N * g.tiles_x * g.H;
@@ -230,8 +233,7 @@ cudaError_t launch_row_t(const CUtensorMap* maps, const GemmArgs& g, cudaStream_
   if (per == 0) return cudaErrorInvalidValue;
   const long long ntiles = (long long)g.N * g.tiles_x * g.H;
   const long long cap = (long long)per * sms, most = ntiles / CR_MIN_TILES;
-  kern<<<(unsigned)(most < cap ? most : cap), 192, smem, s>>>(maps[0], maps[1], g, R);
-  return cudaGetLastError();
+  return launch_pdl(kern, dim3((unsigned)(most < cap ? most : cap)), dim3(192), smem, s, maps[0], maps[1], g, R);
 }
 
 template <int RB>

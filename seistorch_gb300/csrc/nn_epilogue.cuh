@@ -45,7 +45,7 @@ __device__ __forceinline__ void conv_epilogue(const GemmArgs& g, uint32_t taddr,
     const bool whole = co + 16 <= g.Cout;
     if (g.bias != nullptr) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] += (co + j < g.Cout) ? __ldg(g.bias + co + j) : 0.f;
+      for (int j = 0; j < 16; ++j) v[j] += (co + j < g.Cout) ? g.bias[co + j] : 0.f;
     }
     if (g.relu) {
 #pragma unroll
@@ -54,8 +54,8 @@ __device__ __forceinline__ void conv_epilogue(const GemmArgs& g, uint32_t taddr,
     if (g.mask != nullptr) {
       const __nv_bfloat16* mp = g.mask + pix * g.mask_cstride + co;
       if (whole && vm) {
-        const uint4 m0 = __ldg(reinterpret_cast<const uint4*>(mp));
-        const uint4 m1 = __ldg(reinterpret_cast<const uint4*>(mp + 8));
+        const uint4 m0 = *reinterpret_cast<const uint4*>(mp);
+        const uint4 m1 = *reinterpret_cast<const uint4*>(mp + 8);
         const __nv_bfloat16* mb0 = reinterpret_cast<const __nv_bfloat16*>(&m0);
         const __nv_bfloat16* mb1 = reinterpret_cast<const __nv_bfloat16*>(&m1);
 #pragma unroll

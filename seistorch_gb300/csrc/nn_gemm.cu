@@ -136,6 +136,9 @@ __global__ void __launch_bounds__(192, 1) nn_gemm_kernel(const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  // the barriers and the TMEM are set up beside the previous launch
+  pdl_wait();
+  pdl_trigger();
   volatile int* fail = &s_fail;
 
   if (warp == 0) {
@@ -326,8 +329,7 @@ cudaError_t launch_t(const CUtensorMap* maps, const GemmArgs& g0, dim3 grid, cud
   if (ntiles <= 0) return cudaSuccess;
   const long long cap = (long long)per_sm * (sms > 0 ? sms : 152);
   const unsigned nblk = (unsigned)(ntiles < cap ? ntiles : cap);
-  kern<<<nblk, 192, smem, s>>>(maps[0], maps[1], maps[2], maps[3], g);
-  return cudaGetLastError();
+  return launch_pdl(kern, dim3(nblk), dim3(192), smem, s, maps[0], maps[1], maps[2], maps[3], g);
 }
 
 }  // namespace

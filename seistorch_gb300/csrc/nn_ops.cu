@@ -44,8 +44,17 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   }
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
-__device__ __forceinline__ uint4 ld8(const bf16* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
+// Plain loads: the tensors may be what the launch before this one writes, and
+// that launch may still be running when this grid starts (see pdl_wait).
+__device__ __forceinline__ uint4 ld8(const bf16* p) { return *reinterpret_cast<const uint4*>(p); }
 __device__ __forceinline__ void st8(bf16* p, const uint4& v) { *reinterpret_cast<uint4*>(p) = v; }
+
+// Every kernel here is a programmatic dependent of the launch before it (pdl_wait
+// at its start): a prediction is some 16 launches of 4 - 30 us.
+template <class... P, class... A>
+void launch_nn(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A&... args) {
+  launch_pdl(kern, grid, block, smem, s, args...);  // a failure stays for cudaGetLastError
+}
 
 #define GRID_STRIDE(i, total) \
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (total); i += (long long)gridDim.x * blockDim.x)
@@ -57,6 +66,8 @@ __device__ __forceinline__ void st8(bf16* p, const uint4& v) { *reinterpret_cast
 constexpr int TCHW_X = 32;
 __global__ void to_chw_kernel(int n, int h, int w, int c, int cstride, int coff, const bf16* in, int copies,
                               bf16* out) {
+  pdl_wait();
+  pdl_trigger();
   extern __shared__ __align__(16) bf16 tile[];  // [TCHW_X + 2][c]
   const int row = blockIdx.y;  // b * h + y
   const int x0 = blockIdx.x * TCHW_X;
@@ -91,6 +102,8 @@ constexpr int CIN_PX = 4;
 template <bool SMEM_W>
 __global__ void __launch_bounds__(128) conv_in_fwd_kernel(int n, int h, int w, int c, const float* in, const float* W,
                                                           const float* b, bf16* out, int cstride, int coff) {
+  pdl_wait();
+  pdl_trigger();
   // weights of 8 output channels side by side: [c / 8][18 taps + bias][8]
   extern __shared__ __align__(16) float cin_w[];
   if (SMEM_W) {
@@ -150,6 +163,8 @@ __global__ void __launch_bounds__(128) conv_in_fwd_kernel(int n, int h, int w, i
 // Output convolution: c bf16 channels -> 1 fp32 channel (linear).
 __global__ void conv_out_fwd_kernel(int n, int h, int w, int c, const bf16* in, int cstride, const float* W,
                                     const float* b, float* out) {
+  pdl_wait();
+  pdl_trigger();
   const long long total = (long long)n * h * w;
   GRID_STRIDE(i, total) {
     const int x = (int)(i % w);
@@ -184,6 +199,8 @@ constexpr int COUT_TX = 128, COUT_R = 4;
 template <int CV>  // channel vectors per pixel (c = 8 CV)
 __global__ void __launch_bounds__(COUT_TX) conv_out_tile_kernel(int n, int h, int w, const bf16* in, int cstride,
                                                                  const float* W, const float* b, float* out) {
+  pdl_wait();
+  pdl_trigger();
   extern __shared__ __align__(16) unsigned char cout_smem[];
   constexpr int cv = CV, c = 8 * CV, cols = COUT_TX + 2, rows = COUT_R + 2;
   uint4* srow = reinterpret_cast<uint4*>(cout_smem);  // [rows][cols][cv]
@@ -256,6 +273,8 @@ __global__ void __launch_bounds__(COUT_TX) conv_out_tile_kernel(int n, int h, in
 constexpr int COD_PX = 4;
 __global__ void __launch_bounds__(256) conv_out_dgrad_kernel(int n, int h, int w, int c, const float* g, const float* W,
                                                              const bf16* act, int act_cstride, bf16* dx) {
+  pdl_wait();
+  pdl_trigger();
   extern __shared__ __align__(16) float cod_w[];  // [9][c]
   for (int k = threadIdx.x; k < 9 * c; k += blockDim.x) cod_w[k] = W[(k % c) * 9 + k / c];
   __syncthreads();
@@ -322,6 +341,8 @@ template <int SIGN, int NI, bool VEC>
 __global__ void __launch_bounds__(256) vec_scalar_wgrad_kernel(int h, int w, int c, const bf16* v, int v_cstride,
                                                                const float* s, float* dW, float* db_vec,
                                                                float* db_scalar) {
+  pdl_wait();
+  pdl_trigger();
   constexpr int VS_C = 8 / NI, CG = 256 / VS_X;  // channels per thread, channel groups per block
   // the block's part of the images with its halo (0 outside); then the warps' sums
   constexpr int TW = VS_X + 2, TILE = NI * (VS_ROWS + 2) * TW, RED = 8 * CG * (9 * NI + 1) * VS_C;
@@ -344,7 +365,7 @@ __global__ void __launch_bounds__(256) vec_scalar_wgrad_kernel(int h, int w, int
     } else if constexpr (VS_C == 8) {
       unpack8(ok ? ld8(q) : make_uint4(0u, 0u, 0u, 0u), f);
     } else {
-      const uint2 u = ok ? __ldg(reinterpret_cast<const uint2*>(q)) : make_uint2(0u, 0u);
+      const uint2 u = ok ? *reinterpret_cast<const uint2*>(q) : make_uint2(0u, 0u);
       f[0] = __uint_as_float(u.x << 16);
       f[1] = __uint_as_float(u.x & 0xffff0000u);
       f[2] = __uint_as_float(u.y << 16);
@@ -362,7 +383,7 @@ __global__ void __launch_bounds__(256) vec_scalar_wgrad_kernel(int h, int w, int
   for (int q = threadIdx.x; q < TILE; q += 256) {
     const int i = q / ((VS_ROWS + 2) * TW), rr = q / TW % (VS_ROWS + 2), cc = q % TW;
     const int yy = y0 - 1 + rr, xx = blockIdx.x % ntx * VS_X - 1 + cc;
-    sm[q] = (yy >= 0 && yy < h && xx >= 0 && xx < w) ? __ldg(img + i * hw + (long long)yy * w + xx) : 0.f;
+    sm[q] = (yy >= 0 && yy < h && xx >= 0 && xx < w) ? img[i * hw + (long long)yy * w + xx] : 0.f;
   }
   __syncthreads();
   const float* tile = sm + threadIdx.x / CG;
@@ -431,6 +452,8 @@ __global__ void __launch_bounds__(256) vec_scalar_wgrad_kernel(int h, int w, int
 
 // 2x2 average pooling; h, w are the input dims; 8 channels per thread.
 __global__ void pool2_kernel(int n, int h, int w, int c, const bf16* in, int cs_in, int coff_in, bf16* out) {
+  pdl_wait();
+  pdl_trigger();
   const int ho = h / 2, wo = w / 2, cv = c / 8;
   const long long total = (long long)n * ho * wo * cv;
   GRID_STRIDE(i, total) {
@@ -457,6 +480,8 @@ __global__ void pool2_kernel(int n, int h, int w, int c, const bf16* in, int cs_
 // Nearest 2x upsampling into a channel slice; h, w are the output dims;
 // 8 channels per thread.
 __global__ void up2_kernel(int n, int h, int w, int c, const bf16* in, bf16* out, int cs_out, int coff_out) {
+  pdl_wait();
+  pdl_trigger();
   const int cv = c / 8;
   const long long total = (long long)n * h * w * cv;
   GRID_STRIDE(i, total) {
@@ -473,7 +498,7 @@ __global__ void up2_kernel(int n, int h, int w, int c, const bf16* in, bf16* out
 
 // 8 fp32 values of an fp32 gradient (two 16-byte loads).
 __device__ __forceinline__ void ld8f(const float* p, float (&f)[8]) {
-  const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *(reinterpret_cast<const float4*>(p) + 1);
   f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
 }
 
@@ -482,6 +507,8 @@ __device__ __forceinline__ void ld8f(const float* p, float (&f)[8]) {
 // thread.
 __global__ void up2_bwd_kernel(int n, int h, int w, int c, const float* g, int cs_g, int coff_g, const bf16* act,
                                bf16* out) {
+  pdl_wait();
+  pdl_trigger();
   const int ho = h / 2, wo = w / 2, cv = c / 8;
   const long long total = (long long)n * ho * wo * cv;
   GRID_STRIDE(i, total) {
@@ -513,6 +540,8 @@ __global__ void up2_bwd_kernel(int n, int h, int w, int c, const float* g, int c
 // h, w are the fine dims; 8 channels per thread.
 __global__ void pool2_bwd_kernel(int n, int h, int w, int c, const float* gp, const float* gs, int cs_s, int coff_s,
                                  const bf16* act, int cs_a, int coff_a, bf16* out) {
+  pdl_wait();
+  pdl_trigger();
   const int cv = c / 8;
   const long long total = (long long)n * h * w * cv;
   GRID_STRIDE(i, total) {
@@ -542,6 +571,8 @@ __global__ void pool2_bwd_kernel(int n, int h, int w, int c, const float* gp, co
 // db[c] += sum over images and pixels of dy[n][c][p] (channel-major copy);
 // block (split, channel).
 __global__ void bias_grad_kernel(int n, long long hw, int c, const bf16* dy, float* db) {
+  pdl_wait();
+  pdl_trigger();
   const int ch = blockIdx.y;
   float a = 0.f;
   const long long total = (long long)n * hw;
@@ -557,6 +588,8 @@ __global__ void bias_grad_kernel(int n, long long hw, int c, const bf16* dy, flo
 // every blockDim / (c / 8)-th pixel of its block's range, the block's threads of
 // one vector meet in shared memory.
 __global__ void __launch_bounds__(256) bias_grad_nhwc_kernel(long long pixels, int c, const bf16* dy, float* db) {
+  pdl_wait();
+  pdl_trigger();
   extern __shared__ float bsum[];  // [c]
   const int cv = c / 8, per = 256 / cv, v = threadIdx.x % cv, p0 = threadIdx.x / cv;
   for (int k = threadIdx.x; k < c; k += 256) bsum[k] = 0.f;
@@ -579,6 +612,8 @@ __global__ void __launch_bounds__(256) bias_grad_nhwc_kernel(long long pixels, i
 
 // fp32 [cout][cin][3][3] -> bf16 [cout][9][cin] and flipped transpose [cin][9][cout].
 __global__ void pack_weights_kernel(int cout, int cin, const float* W, bf16* wt, bf16* wflip) {
+  pdl_wait();
+  pdl_trigger();
   const long long total = (long long)cout * cin * 9;
   GRID_STRIDE(i, total) {
     const int t = (int)(i % 9);
@@ -592,6 +627,8 @@ __global__ void pack_weights_kernel(int cout, int cin, const float* W, bf16* wt,
 
 __global__ void adam_kernel(long long n, float* p, const float* g, float* m, float* v, float lr, float b1, float b2,
                             float eps, float c1, float c2, float wd) {
+  pdl_wait();
+  pdl_trigger();
   GRID_STRIDE(i, n) {
     const float gi = g[i] + wd * p[i];
     const float mi = b1 * m[i] + (1.f - b1) * gi;
@@ -608,6 +645,8 @@ __global__ void adam_kernel(long long n, float* p, const float* g, float* m, flo
 // and rounded the loss at each of them.
 __global__ void __launch_bounds__(256) mse_kernel(long long n, const float* pred, const float* target, float inv_count,
                                                   float* grad, float* loss) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float part[8];
   float a = 0.f;
   GRID_STRIDE(i, n) {
@@ -634,7 +673,7 @@ cudaError_t launch_to_chw(int n, int h, int w, int c, int cstride, int coff, con
     if (e != cudaSuccess) return e;
   }
   const dim3 grid((unsigned)((w + TCHW_X - 1) / TCHW_X), (unsigned)(n * h));
-  to_chw_kernel<<<grid, 256, smem, s>>>(n, h, w, c, cstride, coff, x, copies, out);
+  launch_nn(to_chw_kernel, grid, 256, smem, s, n, h, w, c, cstride, coff, x, copies, out);
   return cudaGetLastError();
 }
 
@@ -643,9 +682,9 @@ cudaError_t launch_conv_in_fwd(int n, int h, int w, int c, const float* in, cons
   const long long threads = (long long)n * h * ((w + CIN_PX - 1) / CIN_PX);
   const int blocks = blocks_for(2 * threads);
   if (c <= 256)
-    conv_in_fwd_kernel<true><<<blocks, 128, (size_t)19 * c * 4, s>>>(n, h, w, c, in, W, b, out, cstride, coff);
+    launch_nn(conv_in_fwd_kernel<true>, blocks, 128, (size_t)19 * c * 4, s, n, h, w, c, in, W, b, out, cstride, coff);
   else
-    conv_in_fwd_kernel<false><<<blocks, 128, 0, s>>>(n, h, w, c, in, W, b, out, cstride, coff);
+    launch_nn(conv_in_fwd_kernel<false>, blocks, 128, 0, s, n, h, w, c, in, W, b, out, cstride, coff);
   return cudaGetLastError();
 }
 
@@ -659,7 +698,7 @@ cudaError_t launch_conv_in_wgrad(int n, int h, int w, int c, const float* in, co
   const dim3 grid((unsigned)vs_blocks(n, h, w), (unsigned)((c + 15) / 16));
   const bool vec = c % 4 == 0 && dy_cstride % 4 == 0 && (reinterpret_cast<uintptr_t>(dy) & 7u) == 0;
   auto kern = vec ? vec_scalar_wgrad_kernel<1, 2, true> : vec_scalar_wgrad_kernel<1, 2, false>;
-  kern<<<grid, 256, 0, s>>>(h, w, c, dy, dy_cstride, in, dW, db, nullptr);
+  launch_nn(kern, grid, 256, 0, s, h, w, c, dy, dy_cstride, in, dW, db, nullptr);
   return cudaGetLastError();
 }
 
@@ -675,10 +714,10 @@ cudaError_t launch_conv_out_fwd(int n, int h, int w, int c, const bf16* in, int 
       set[c == 64] = true;
     }
     const long long blocks = (long long)n * ((h + COUT_R - 1) / COUT_R) * ((w + COUT_TX - 1) / COUT_TX);
-    kern<<<(unsigned)blocks, COUT_TX, smem, s>>>(n, h, w, in, cstride, W, b, out);
+    launch_nn(kern, (unsigned)blocks, COUT_TX, smem, s, n, h, w, in, cstride, W, b, out);
     return cudaGetLastError();
   }
-  conv_out_fwd_kernel<<<blocks_for((long long)n * h * w), 256, 0, s>>>(n, h, w, c, in, cstride, W, b, out);
+  launch_nn(conv_out_fwd_kernel, blocks_for((long long)n * h * w), 256, 0, s, n, h, w, c, in, cstride, W, b, out);
   return cudaGetLastError();
 }
 
@@ -689,44 +728,44 @@ cudaError_t launch_conv_out_bwd(int n, int h, int w, int c, const float* g, cons
     cudaError_t e = cudaFuncSetAttribute(conv_out_dgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  conv_out_dgrad_kernel<<<blocks_for((long long)n * h * ((w + COD_PX - 1) / COD_PX) * (c / 8)), 256, smem, s>>>(
-      n, h, w, c, g, W, act, act_cstride, dx);
+  launch_nn(conv_out_dgrad_kernel, blocks_for((long long)n * h * ((w + COD_PX - 1) / COD_PX) * (c / 8)), 256, smem, s,
+            n, h, w, c, g, W, act, act_cstride, dx);
   // 4 channel groups of 8 channels per block
   const dim3 grid((unsigned)vs_blocks(n, h, w), (unsigned)((c + 31) / 32));
-  vec_scalar_wgrad_kernel<-1, 1, true><<<grid, 256, 0, s>>>(h, w, c, act, act_cstride, g, dW, nullptr, db);
+  launch_nn(vec_scalar_wgrad_kernel<-1, 1, true>, grid, 256, 0, s, h, w, c, act, act_cstride, g, dW, nullptr, db);
   return cudaGetLastError();
 }
 
 cudaError_t launch_pool2(int n, int h, int w, int c, const bf16* in, int cs_in, int coff_in, bf16* out,
                          cudaStream_t s) {
-  pool2_kernel<<<blocks_for((long long)n * (h / 2) * (w / 2) * (c / 8)), 256, 0, s>>>(n, h, w, c, in, cs_in, coff_in,
-                                                                                     out);
+  launch_nn(pool2_kernel, blocks_for((long long)n * (h / 2) * (w / 2) * (c / 8)), 256, 0, s,
+            n, h, w, c, in, cs_in, coff_in, out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_up2(int n, int h, int w, int c, const bf16* in, bf16* out, int cs_out, int coff_out,
                        cudaStream_t s) {
-  up2_kernel<<<blocks_for((long long)n * h * w * (c / 8)), 256, 0, s>>>(n, h, w, c, in, out, cs_out, coff_out);
+  launch_nn(up2_kernel, blocks_for((long long)n * h * w * (c / 8)), 256, 0, s, n, h, w, c, in, out, cs_out, coff_out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_up2_bwd(int n, int h, int w, int c, const float* g, int cs_g, int coff_g, const bf16* act,
                            bf16* out, cudaStream_t s) {
-  up2_bwd_kernel<<<blocks_for((long long)n * (h / 2) * (w / 2) * (c / 8)), 256, 0, s>>>(n, h, w, c, g, cs_g, coff_g,
-                                                                                         act, out);
+  launch_nn(up2_bwd_kernel, blocks_for((long long)n * (h / 2) * (w / 2) * (c / 8)), 256, 0, s,
+            n, h, w, c, g, cs_g, coff_g, act, out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_pool2_bwd(int n, int h, int w, int c, const float* gp, const float* gs, int cs_s, int coff_s,
                              const bf16* act, int cs_a, int coff_a, bf16* out, cudaStream_t s) {
-  pool2_bwd_kernel<<<blocks_for((long long)n * h * w * (c / 8)), 256, 0, s>>>(n, h, w, c, gp, gs, cs_s, coff_s, act,
-                                                                               cs_a, coff_a, out);
+  launch_nn(pool2_bwd_kernel, blocks_for((long long)n * h * w * (c / 8)), 256, 0, s,
+            n, h, w, c, gp, gs, cs_s, coff_s, act, cs_a, coff_a, out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_bias_grad(int n, long long hw, int c, const bf16* dy, float* db, cudaStream_t s) {
   const dim3 grid(32, c);
-  bias_grad_kernel<<<grid, 256, 0, s>>>(n, hw, c, dy, db);
+  launch_nn(bias_grad_kernel, grid, 256, 0, s, n, hw, c, dy, db);
   return cudaGetLastError();
 }
 
@@ -734,26 +773,26 @@ cudaError_t launch_bias_grad_nhwc(long long pixels, int c, const bf16* dy, float
   if (c > 2048) return cudaErrorInvalidValue;  // one channel vector per thread
   long long b = (pixels * (c / 8) + 256 * 32 - 1) / (256 * 32);
   b = b > 152 * 8 ? 152 * 8 : b;
-  bias_grad_nhwc_kernel<<<(unsigned)b, 256, (size_t)c * 4, s>>>(pixels, c, dy, db);
+  launch_nn(bias_grad_nhwc_kernel, (unsigned)b, 256, (size_t)c * 4, s, pixels, c, dy, db);
   return cudaGetLastError();
 }
 
 cudaError_t launch_pack_weights(int cout, int cin, const float* W, bf16* wt, bf16* wflip, cudaStream_t s) {
-  pack_weights_kernel<<<blocks_for((long long)cout * cin * 9), 256, 0, s>>>(cout, cin, W, wt, wflip);
+  launch_nn(pack_weights_kernel, blocks_for((long long)cout * cin * 9), 256, 0, s, cout, cin, W, wt, wflip);
   return cudaGetLastError();
 }
 
 cudaError_t launch_adam(long long n, float* p, const float* g, float* m, float* v, float lr, float b1, float b2,
                         float eps, int step, float wd, cudaStream_t s) {
   const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
-  adam_kernel<<<blocks_for(n), 256, 0, s>>>(n, p, g, m, v, lr, b1, b2, eps, c1, c2, wd);
+  launch_nn(adam_kernel, blocks_for(n), 256, 0, s, n, p, g, m, v, lr, b1, b2, eps, c1, c2, wd);
   return cudaGetLastError();
 }
 
 cudaError_t launch_mse(long long n, const float* pred, const float* target, float* grad, float* loss,
                        cudaStream_t s) {
   const int b = blocks_for(n);
-  mse_kernel<<<b < 152 * 4 ? b : 152 * 4, 256, 0, s>>>(n, pred, target, 1.f / (float)n, grad, loss);
+  launch_nn(mse_kernel, b < 152 * 4 ? b : 152 * 4, 256, 0, s, n, pred, target, 1.f / (float)n, grad, loss);
   return cudaGetLastError();
 }
 

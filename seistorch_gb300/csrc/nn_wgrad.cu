@@ -85,6 +85,9 @@ __global__ void __launch_bounds__(128) nn_wgrad_kernel(const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  // the barriers and the TMEM are set up beside the previous launch
+  pdl_wait();
+  pdl_trigger();
   volatile int* fail = &s_fail;
   constexpr int GROUPS = 9 / TAPS;  // tap rows, or single taps
   const int tap0 = (blockIdx.y % GROUPS) * TAPS, ky = tap0 / 3, kx0 = tap0 - 3 * ky;
@@ -198,8 +201,7 @@ cudaError_t launch_s(const CUtensorMap* maps, const WgradArgs& g, int splits, cu
     set = true;
   }
   const dim3 grid((unsigned)splits, (unsigned)(9 / TAPS * ((g.Cin + 127) / 128)), (unsigned)((g.Cout + BN - 1) / BN));
-  kern<<<grid, 128, Lay::BYTES, s>>>(maps[0], maps[1], g);
-  return cudaGetLastError();
+  return launch_pdl(kern, dim3(grid), dim3(128), Lay::BYTES, s, maps[0], maps[1], g);
 }
 
 template <int BN, int TAPS>
