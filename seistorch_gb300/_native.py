@@ -290,12 +290,19 @@ def check(status, what):
         raise NativeError(f"{what} failed: {msg}{extra}")
 
 
+_FN = {}  # entry points by name, filled on first use (the library is never unloaded)
+
+
 def call(name, *args):
-    lib = load()
-    fn = getattr(lib, name, None)
+    fn = _FN.get(name)
     if fn is None:
-        raise NativeError(f"{LIB_NAME} does not export {name}")
-    check(fn(*args), name)
+        fn = getattr(load(), name, None)
+        if fn is None:
+            raise NativeError(f"{LIB_NAME} does not export {name}")
+        _FN[name] = fn
+    status = fn(*args)
+    if status != 0:
+        check(status, name)
 
 
 SCHEME_ACOUSTIC = 0   # 2nd-order-in-time cross-stencil family (acoustic, HABC, Born, VTI, density)
@@ -333,5 +340,11 @@ def ptr(t):
 
 
 def stream_handle(device=None):
+    """The current CUDA stream as a raw handle.  A time step or a layer of the
+    preconditioner is a call of a few microseconds; torch.cuda.current_stream()
+    builds a Stream object on each (4 to 6 us)."""
     import torch
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if raw is None or device is not None:
+        return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    return ctypes.c_void_p(raw(torch.cuda.current_device()))

@@ -293,9 +293,8 @@ class AcousticPropagator:
         dJ/dvp over the whole grid (k = vp^2 dt^2 / h^2, so dk/dvp = 2 vp dt^2 / h^2)."""
         m, keep = self.model(vp, damp, blend)
         r = self.habc_vjp(m, u, um, gy)
-        gvp = r["gparam"][0] * (2.0 * (self.dt / self.h) ** 2) * vp.detach().to(torch.float32)
-        if blend:
-            gvp = gvp + r["gc"]
+        scale, v = 2.0 * (self.dt / self.h) ** 2, vp.detach().to(torch.float32)
+        gvp = torch.addcmul(r["gc"], r["gparam"][0], v, value=scale) if blend else r["gparam"][0] * scale * v
         return r["gu"], r["gum"], gvp
 
     # -- whole loop

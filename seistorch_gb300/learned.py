@@ -37,6 +37,7 @@ from . import _native as N
 LAYERS = [("e1a", 2, 32, "in"), ("e1b", 32, 32, "tc"), ("e2a", 32, 64, "tc"), ("e2b", 64, 64, "tc"),
           ("e3a", 64, 128, "tc"), ("e3b", 128, 128, "tc"), ("b4", 128, 256, "tc"), ("d3", 384, 128, "tc"),
           ("d2", 192, 64, "tc"), ("d1", 96, 32, "tc"), ("out", 32, 1, "out")]
+SHAPE = {name: (ci, co) for name, ci, co, _ in LAYERS}
 BF16 = torch.bfloat16
 
 
@@ -124,21 +125,21 @@ class PrecondNet:
 
     # -- layers
     def _tc(self, name, x, h, w, out, cstride, coff, relu=True, bias=True):
-        _, ci, co, _ = next(l for l in LAYERS if l[0] == name)
+        ci, co = SHAPE[name]
         B = self._shape[0]
         c = N.NnConv(B, h, w, ci, co, N.ptr(x), N.ptr(self.wt[name]), N.ptr(self.b[name]) if bias else None,
                      int(relu), None, 0, N.ptr(out), None, cstride, coff)
         N.call("sgb_nn_conv3x3", ctypes.byref(c), N.stream_handle())
 
     def _tc_dgrad(self, name, dy, h, w, out_f32=None, out_bf16=None, mask=None):
-        _, ci, co, _ = next(l for l in LAYERS if l[0] == name)
+        ci, co = SHAPE[name]
         B = self._shape[0]
         c = N.NnConv(B, h, w, co, ci, N.ptr(dy), N.ptr(self.wflip[name]), None, 0, N.ptr(mask),
                      ci if mask is not None else 0, N.ptr(out_bf16), N.ptr(out_f32), ci, 0)
         N.call("sgb_nn_conv3x3", ctypes.byref(c), N.stream_handle())
 
     def _tc_wgrad(self, name, dy, x, h, w):
-        _, ci, co, _ = next(l for l in LAYERS if l[0] == name)
+        ci, co = SHAPE[name]
         B = self._shape[0]
         s = N.stream_handle()
         p = N.NnWgradNhwc(B, h, w, ci, co, N.ptr(dy), N.ptr(x), N.ptr(self.gW[name]))

@@ -163,6 +163,7 @@ class WaveRNN(torch.nn.Module):
             raise NotImplementedError(f"equation '{eq}' is not implemented by seistorch_gb300")
         if self.source_illumination:
             self.precondition = illum
-        y = TensorList(torch.split(rec, reccounts, dim=1))
-        y.has_nan()
-        return y
+        # NaN check (rnn.py:215) on the records of the whole batch: one device read
+        # instead of one per shot
+        TensorList([rec.detach()]).has_nan()
+        return TensorList(torch.split(rec, reccounts, dim=1))
