@@ -57,8 +57,10 @@ __global__ void __launch_bounds__(32 * NWP, TZ / NWP <= 2 ? (PTM >= 2 ? 3 : 4) :
   const int ntiles = a.nshots * a.ntx * a.nzc;
   const int G = gridDim.x;
 
-  auto issue = [&](int t, int stage) {
-    const Tile g = tile_geom(t, a.nshots, a.ntx, TZ);
+  TileWalk walk(blockIdx.x, G, a.nshots, a.ntx, TZ), ahead = walk;  // this tile, the next one to load
+  auto issue = [&](int stage) {
+    const Tile g = ahead.g;
+    ahead.next(TZ);
     float* st = smem + stage * Lay::STAGE;
     fence_proxy_async_smem();
     mbar_arrive_expect_tx(&bars[stage], Lay::TX_BYTES);
@@ -80,16 +82,16 @@ __global__ void __launch_bounds__(32 * NWP, TZ / NWP <= 2 ? (PTM >= 2 ? 3 : 4) :
   pdl_trigger();
   if (tid == 0)
     for (int s = 0; s < S; ++s)
-      if ((int)blockIdx.x + s * G < ntiles) issue(blockIdx.x + s * G, s);
+      if ((int)blockIdx.x + s * G < ntiles) issue(s);
   // the saved ring of U_{j-2}, each CTA a share while its first boxes load:
   // the tiles never write ring cells, and nothing in this launch reads U_{j-2}
   if (a.do_recon && a.ring_in != nullptr)
     ring_copy_share(a.ring, a.nshots, a.pitch, a.sstride, a.uout, const_cast<float*>(a.ring_in), true);
   __syncthreads();
   int k = 0;
-  for (int t = blockIdx.x; t < ntiles; t += G, ++k) {
+  for (int t = blockIdx.x; t < ntiles; t += G, ++k, walk.next(TZ)) {
     const int stage = k % S;
-    const Tile g = tile_geom(t, a.nshots, a.ntx, TZ);
+    const Tile g = walk.g;
     const int x = g.x0 + 4 * lane;
     const bool xin = x < a.nx;
     const int zw = g.z0 + wid * RPW;
@@ -213,7 +215,7 @@ __global__ void __launch_bounds__(32 * NWP, TZ / NWP <= 2 ? (PTM >= 2 ? 3 : 4) :
       }
     }
     if (__syncthreads_or(s_abort)) break;  // stage free
-    if (tid == 0 && t + S * G < ntiles) issue(t + S * G, stage);
+    if (tid == 0 && t + S * G < ntiles) issue(stage);
   }
   if (s_abort && tid == 0)
     for (int q = k; q < k + S; ++q)

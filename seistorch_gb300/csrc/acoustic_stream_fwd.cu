@@ -118,6 +118,12 @@ struct FwdTileLayout {
 // numbered group after group from tile0[g].
 template <int SB>
 struct FwdOne {
+  static constexpr bool ONE = true;
+  using Walk = TileWalk;
+  template <int>
+  __device__ __forceinline__ Walk walk(int t, int G, int tz) const {
+    return TileWalk(t, G, (a.nshots + SB - 1) / SB, a.ntx, tz);
+  }
   const CUtensorMap* tu;
   const CUtensorMap* tum;
   AcStreamArgs a;
@@ -131,6 +137,10 @@ struct FwdOne {
 
 template <int MAXG>
 struct FwdMany {
+  static constexpr bool ONE = false;
+  struct Walk {};
+  template <int>
+  __device__ __forceinline__ Walk walk(int, int, int) const { return {}; }
   const AcFwdBatch<MAXG>& B;
   __device__ __forceinline__ int ntiles() const { return B.tile0[B.ngroups]; }
   __device__ __forceinline__ int group(int t) const {
@@ -169,10 +179,20 @@ __device__ __forceinline__ void fwd_tiles(const P& prov, const Pre& pre = Pre{})
   const int ntiles = prov.ntiles();
   const int G = gridDim.x;
 
+  // tile geometry: a walk without divisions on one grid, per tile over several
+  typename P::Walk walk = prov.template walk<SB>(blockIdx.x, G, TZ), ahead = walk;  // this tile, the next one to load
+  auto geom = [&](typename P::Walk& w, int t, int gi, const AcStreamArgs& a) -> Tile {
+    if constexpr (P::ONE) {
+      const Tile g = w.g;
+      w.next(TZ);
+      return g;
+    } else {
+      return tile_geom(t - prov.first(gi), (a.nshots + SB - 1) / SB, a.ntx, TZ);
+    }
+  };
   auto issue = [&](int t, int stage) {
     const int gi = prov.group(t);
-    const AcStreamArgs& a = prov.args(gi);
-    const Tile g = tile_geom(t - prov.first(gi), (a.nshots + SB - 1) / SB, a.ntx, TZ);
+    const Tile g = geom(ahead, t, gi, prov.args(gi));
     fence_proxy_async_smem();
     mbar_arrive_expect_tx(&bars[stage], Lay::TX_BYTES);
     tma_load_3d(smem + stage * Lay::STAGE, prov.map_u(gi), g.x0 - LO, g.z0 - R, g.b * SB, &bars[stage]);
@@ -196,7 +216,7 @@ __device__ __forceinline__ void fwd_tiles(const P& prov, const Pre& pre = Pre{})
     const int stage = k % S;
     const int gi = prov.group(t);
     const AcStreamArgs& a = prov.args(gi);
-    const Tile g = tile_geom(t - prov.first(gi), (a.nshots + SB - 1) / SB, a.ntx, TZ);
+    const Tile g = geom(walk, t, gi, a);
     const int x = g.x0 + 4 * lane;
     const bool xin = x < a.nx;
     const int zw = g.z0 + wid * RPW;  // first row of this warp

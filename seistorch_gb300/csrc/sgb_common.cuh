@@ -37,6 +37,37 @@ __device__ __forceinline__ void set_comp(float4& v, int m, float a) {
   if (m == 0) v.x = a; else if (m == 1) v.y = a; else if (m == 2) v.z = a; else v.w = a;
 }
 
+// Two adjacent floats as one packed operand: add / fma of both halves in one
+// instruction, each rounded as the scalar operation is.
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack(F2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+  return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+
 // Bytes of a 16-byte chunk starting at column x of a row of nx valid floats
 // (0 outside [0, nx): zero fill == the zero padding of conv2d / roll edges).
 __device__ __forceinline__ int chunk_bytes(int z, int x, int nz, int nx) {

@@ -37,7 +37,7 @@ struct Row {
   static constexpr int LO = (W - TX) / 2;
 };
 
-// Tile t -> (shot, strip, band); 32-bit arithmetic.
+// Tile t -> (shot, strip, band), shot fastest; 32-bit arithmetic.
 struct Tile {
   int b, x0, z0;
 };
@@ -49,6 +49,28 @@ __device__ __forceinline__ Tile tile_geom(int t, int nshots, int ntx, int tz) {
   g.z0 = (rest / ntx) * tz;
   return g;
 }
+// The same for the tiles t, t + G, t + 2 G, ... of a CTA without a division per
+// tile: (shot, strip, band) advance by those of G, with carries.
+struct TileWalk {
+  Tile g;      // of the current tile
+  Tile d;      // of G
+  int nshots, nx;  // carry limits: shots, ntx * TX
+  __device__ __forceinline__ TileWalk(int t, int G, int nshots_, int ntx, int tz)
+      : g(tile_geom(t, nshots_, ntx, tz)), d(tile_geom(G, nshots_, ntx, tz)), nshots(nshots_), nx(ntx * TX) {}
+  __device__ __forceinline__ void next(int tz) {
+    g.b += d.b;
+    g.x0 += d.x0;
+    g.z0 += d.z0;
+    if (g.b >= nshots) {
+      g.b -= nshots;
+      g.x0 += TX;
+    }
+    if (g.x0 >= nx) {
+      g.x0 -= nx;
+      g.z0 += tz;
+    }
+  }
+};
 
 __device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
 
@@ -62,7 +84,10 @@ __device__ __forceinline__ float gather_lane(const float4& v, int rx) {
 
 // Cross-stencil Laplacian (without 1/h^2) of the 4 columns of a lane at the
 // centre row of `win`, x-neighbours from the staged row `srow` (its element
-// Row<R>::LO is column x0).
+// Row<R>::LO is column x0).  Two columns per instruction: the tile kernels are
+// bound by how many instructions their 16 warps per SM issue (427 per 128-point
+// row of the 8th-order adjoint, half of the issue slots).  With the division-free
+// walk above: 64 shots of 500 x 1100, 160 steps and their adjoint 44.7 -> 42.8 ms.
 template <int R>
 __device__ __forceinline__ float4 lap_row(const float4 (&win)[2 * R + 1], const float* srow, int lane,
                                           const FdWeights& w) {
@@ -70,16 +95,24 @@ __device__ __forceinline__ float4 lap_row(const float4 (&win)[2 * R + 1], const 
   const float4 r = lds4(srow + Row<R>::LO + 4 + 4 * lane);
   const float4 c = win[R];
   const float a[12] = {l.x, l.y, l.z, l.w, c.x, c.y, c.z, c.w, r.x, r.y, r.z, r.w};
-  float4 L;
+  float2 o[2];
 #pragma unroll
-  for (int m = 0; m < 4; ++m) {
-    float s = w.c[0] * a[4 + m];
+  for (int h = 0; h < 2; ++h) {  // columns 2h, 2h + 1
+    const int m = 4 + 2 * h;
+    F2 s = mul2(f2(w.c[0], w.c[0]), f2(a[m], a[m + 1]));
 #pragma unroll
-    for (int j = 1; j <= R; ++j)
-      s = fmaf(w.c[j], (a[4 + m + j] + a[4 + m - j]) + (comp(win[R + j], m) + comp(win[R - j], m)), s);
-    set_comp(L, m, s);
+    for (int j = 1; j <= R; ++j) {
+      const float4 &u = win[R + j], &d = win[R - j];
+      // odd offsets straddle the register pairs of the loaded quads: scalar sums
+      // (written as a pair) cost less than the moves that would pair their operands
+      const F2 xs = (j & 1) ? f2(a[m + j] + a[m - j], a[m + 1 + j] + a[m + 1 - j])
+                            : add2(f2(a[m + j], a[m + 1 + j]), f2(a[m - j], a[m + 1 - j]));
+      const F2 zs = h == 0 ? add2(f2(u.x, u.y), f2(d.x, d.y)) : add2(f2(u.z, u.w), f2(d.z, d.w));
+      s = fma2(f2(w.c[j], w.c[j]), add2(xs, zs), s);
+    }
+    o[h] = unpack(s);
   }
-  return L;
+  return make_float4(o[0].x, o[0].y, o[1].x, o[1].y);
 }
 
 // Sources of shot b in rows [zlo, zlo + nrow) and columns [x0, x0 + 128):
