@@ -30,6 +30,8 @@
 // (C D(U), acoustic_rho_habc.py) and Born (the scattered field's adjoint
 // against the background's reconstruction, acoustic_lsrtm_habc.py)
 // gradients.
+#include <type_traits>
+
 #include "sgb_common.cuh"
 #include "acoustic_args.cuh"
 
@@ -78,6 +80,7 @@ struct HabcBwdArgs {
   // block of far tiles, strips [fx0, fx1) x bands [fz0, fz1): the far
   // launch covers that block, the near launch the frame around it
   int ntx, nzb, fx0, fx1, fz0, fz1;
+  int nfar, nnear;  // tiles of each kind per shot
   long long sstride;
   const float* __restrict__ la1;   // La_{j+1}
   const float* __restrict__ la2;   // La_{j+2}
@@ -388,25 +391,52 @@ __global__ void __launch_bounds__(256) habc_step_vjp_kernel(const HabcVjpArgs a)
 // habc_shares_kernel fills once per reverse loop; then the receiver
 // residuals, the gradient term and the reconstruction inside the box, the
 // saved ring (or 0) outside it.
+
+// Cross-stencil Laplacian of the cells (rr, cx .. cx + 3) of a shared tile, two
+// columns per instruction.
+template <int R, int W>
+__device__ __forceinline__ float4 lap_rows4(const float (*s)[W], int rr, int cx, const FdWeights& w) {
+  const float4 l = lds4(&s[rr][cx - 4]), c = lds4(&s[rr][cx]), r = lds4(&s[rr][cx + 4]);
+  const float a[12] = {l.x, l.y, l.z, l.w, c.x, c.y, c.z, c.w, r.x, r.y, r.z, r.w};
+  F2 o[2] = {mul2(f2(w.c[0], w.c[0]), f2(c.x, c.y)), mul2(f2(w.c[0], w.c[0]), f2(c.z, c.w))};
+#pragma unroll
+  for (int j = 1; j <= R; ++j) {
+    const float4 d = lds4(&s[rr - j][cx]), u = lds4(&s[rr + j][cx]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int m = 4 + 2 * h;
+      const F2 xs = (j & 1) ? f2(a[m + j] + a[m - j], a[m + 1 + j] + a[m + 1 - j])
+                            : add2(f2(a[m + j], a[m + 1 + j]), f2(a[m - j], a[m + 1 - j]));
+      const F2 zs = h == 0 ? add2(f2(u.x, u.y), f2(d.x, d.y)) : add2(f2(u.z, u.w), f2(d.z, d.w));
+      o[h] = fma2(f2(w.c[j], w.c[j]), add2(xs, zs), o[h]);
+    }
+  }
+  const float2 p = unpack(o[0]), q = unpack(o[1]);
+  return make_float4(p.x, p.y, q.x, q.y);
+}
+
 template <int R, int EQ, bool NEAR>
-__device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a) {
+__device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a, int tile) {
   constexpr bool VTI = EQ == 1, RHO = EQ == 2;
   static_assert(!RHO || R == 1, "variable density is second order");
-  // row halo: the stencil's R, and 2 for the one-way lines (q - d, q - 2d)
-  constexpr int HR = R < 2 ? 2 : R;
+  // row halo: the stencil's R, and 2 for the one-way lines (q - d, q - 2d) near a strip
+  constexpr int HN = R < 2 ? 2 : R, HR = NEAR ? HN : R;
   constexpr int ROWS = HT_Z + 2 * HR, W = HT_X + 2 * HT_H;
   __shared__ __align__(16) float s_kl[ROWS][W];             // k wi La1 (VTI: kx wi La1; density: C wi La1)
   __shared__ __align__(16) float s_kzl[VTI ? ROWS : 1][W];  // VTI: kz wi La1
   __shared__ __align__(16) float s_u[ROWS][W];
   __shared__ __align__(16) float s_l1[NEAR ? ROWS : 1][W];  // La1 and La2 (tiles near a strip only)
   __shared__ __align__(16) float s_l2[NEAR ? ROWS : 1][W];
-  const int b = blockIdx.z;
+  // tile of this kind -> (shot, band, strip), strips fastest
+  const int ntile = NEAR ? a.nnear : a.nfar;
+  const int b = tile / ntile;
+  int i = tile - b * ntile;
   int strip, band;
   if constexpr (!NEAR) {
-    strip = a.fx0 + (int)blockIdx.x;
-    band = a.fz0 + (int)blockIdx.y;
+    const int nf = a.fx1 - a.fx0;
+    band = a.fz0 + i / nf;
+    strip = a.fx0 + i % nf;
   } else {  // the frame: the bands above the far block, the strips beside it, the bands below
-    int i = blockIdx.x;
     const int top = a.fz0 * a.ntx, nside = a.ntx - (a.fx1 - a.fx0), mid = (a.fz1 - a.fz0) * nside;
     if (i < top) {
       band = i / a.ntx;
@@ -424,8 +454,10 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a) {
   }
   const int z0 = band * HT_Z, x0 = strip * HT_X;
   const long long fb = (long long)b * a.sstride;
-  const float* l1 = a.la1 + fb;
-  const float* u1 = a.ujm1 + fb;
+  const float* l1 = after_wait(a.la1 + fb);
+  const float* l2 = after_wait(a.la2 + fb);
+  const float* u1 = after_wait(a.ujm1 + fb);
+  const float* u0 = after_wait(a.uj + fb);
   const int tid = threadIdx.y * 32 + threadIdx.x;
   const int hw = a.hw;
   const bool mult = a.multiple != 0;
@@ -433,7 +465,7 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a) {
   const float* __restrict__ kp = RHO ? a.rho_c : a.k;  // the plane that weights La1
   // does any cell of the tile or its halo have an interior share below 1, or
   // lie within reach of a one-way line (depth <= hw)?
-  const bool near = hw > 0 && ((!mult && z0 - HR <= hw) || z0 + HT_Z + HR >= a.nz - 1 - hw ||
+  const bool near = hw > 0 && ((!mult && z0 - HN <= hw) || z0 + HT_Z + HN >= a.nz - 1 - hw ||
                                 x0 - HT_H <= hw || x0 + HT_X + HT_H >= a.nx - 1 - hw);
   // two launches share the grid: the NEAR instantiation takes the tiles
   // within reach of a strip, the other the rest (with none of the strip code)
@@ -470,10 +502,10 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a) {
     if (c < NST && zs >= 0 && zs < a.nz && xs >= 0 && xs < a.nx) {
       const long long os = (long long)zs * a.pitch + xs;
       g.k = __ldg(reinterpret_cast<const float4*>(kp + os));
-      g.l = ldf4(l1 + os);
+      g.l = ld4(l1 + os);
       if (VTI) g.q = __ldg(reinterpret_cast<const float4*>(a.kz + os));
-      g.v = ldf4(u1 + os);
-      if (NEAR) g.m = ldf4(a.la2 + fb + os);
+      g.v = ld4(u1 + os);
+      if (NEAR) g.m = ld4(l2 + os);
       if (NEAR) g.w = wi4_at(zs, xs);
     }
   };
@@ -513,14 +545,14 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a) {
     k4 = __ldg(reinterpret_cast<const float4*>(kp + o));
     if (VTI) kz4 = __ldg(reinterpret_cast<const float4*>(a.kz + o));
     if (!NEAR) {
-      l2g = ldf4(a.la2 + fb + o);
-      l1g = ldf4(l1 + o);
+      l2g = ld4(l2 + o);
+      l1g = ld4(l1 + o);
     }
   };
   // U_j of the four cells (reconstruction)
   auto tail_loads = [&]() {
     if (!cell_in) return;
-    if (a.uout != nullptr && row_in) uj4 = ldf4(a.uj + fb + o);
+    if (a.uout != nullptr && row_in) uj4 = ld4(u0 + o);
   };
   if constexpr (PRE) {
     Grp g[NIT];
@@ -561,9 +593,6 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a) {
     if (x > 0) bxpL = __ldg(a.rho_c + pl + o - 1);
     if (x + 4 < a.nx) bxnR = __ldg(a.rho_c + 2 * pl + o + 4);
   }
-  // one-way transposes of side `sd` at cell (z, xm) of local column cxm:
-  // strip cells p = q, q - d, q - 2d (staged La1 / La2) and the wrap of the
-  // line's depth hw-1 cell into its edge cell (global)
   auto share = [&](int sd, int pz, int px) -> float {
     const long long oo = (long long)pz * a.pitch + px;
     if (a.wpl != nullptr) return __ldg(a.wpl + (1 + sd) * pl + oo);
@@ -572,46 +601,62 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a) {
     const HabcW w = habc_weights(pz, px, a.nz, a.nx, hw, mult, bb);
     return sd == 0 ? w.wt : sd == 1 ? w.wb : sd == 2 ? w.wl : w.wr;
   };
-  auto oneway = [&](int sd, int dq, int sz, int sx, int xm, int cxm) -> float {
-    if (dq > hw) return 0.f;
-    float acc = 0.f;
-    if (dq < hw) {
-      const float ws = share(sd, z, xm);
-      if (ws != 0.f) {
-        const float c = __ldg(a.vp + (long long)z * a.pitch + xm);
-        const float lam = c * a.lamf, mu = c * c * a.muf;
-        acc += ws * ((2.f - lam - mu) * s_l1[rr][cxm] + (lam - 1.f) * s_l2[rr][cxm]);
+  // one-way transposes of the left (SX = 1) or right (SX = -1) side at the
+  // lane's four cells: strip cells p = q, q - d, q - 2d (staged La1 / La2), whose
+  // columns are the lane's group and the one before it along d, so that shares
+  // and velocities are two 16-byte rows (a cell beyond the strip has share 0),
+  // and the wrap of the line's depth hw-1 cell into its edge cell (global).
+  // Cell by cell, the strips' warps issued about 1200 instructions per row.
+  auto share_cols = [&](int sd, int px) -> float4 {
+    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (px < 0 || px >= a.nx) return r;
+    if (a.wpl != nullptr)
+      return __ldg(reinterpret_cast<const float4*>(a.wpl + (1 + sd) * pl + (long long)z * a.pitch + px));
+#pragma unroll 1
+    for (int m = 0; m < 4; ++m)
+      if (px + m < a.nx) set_comp(r, m, share(sd, z, px + m));
+    return r;
+  };
+  auto vp_cols = [&](int px) -> float4 {
+    if (px < 0 || px >= a.nx) return make_float4(0.f, 0.f, 0.f, 0.f);
+    return __ldg(reinterpret_cast<const float4*>(a.vp + (long long)z * a.pitch + px));
+  };
+  auto oneway_cols = [&](auto dir, float4& acc) {
+    constexpr int SX = decltype(dir)::value;
+    constexpr int sd = SX > 0 ? 2 : 3;
+    const float4 w0 = share_cols(sd, x), w1 = share_cols(sd, x - 4 * SX);
+    const float4 c0 = vp_cols(x), c1 = vp_cols(x - 4 * SX);
+    // entry i: strip cell x + i for SX = 1 (i = -2 .. 3), x + 3 - i for SX = -1
+    auto at = [&](const float4& g0, const float4& g1, int i) -> float {
+      return SX > 0 ? (i >= 0 ? comp(g0, i) : comp(g1, 4 + i)) : (i >= 0 ? comp(g0, 3 - i) : comp(g1, -1 - i));
+    };
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {  // the cell at entry i
+      const int m = SX > 0 ? i : 3 - i, xm = x + m, dq = SX > 0 ? xm : a.nx - 1 - xm;
+      float t = 0.f;
+      {
+        const float ws = at(w0, w1, i), c = at(c0, c1, i), lam = c * a.lamf, mu = c * c * a.muf;
+        t += ws * ((2.f - lam - mu) * s_l1[rr][cx + m] + (lam - 1.f) * s_l2[rr][cx + m]);
       }
-    }
-    if (dq >= 1) {
-      const int pz = z - sz, px = xm - sx;
-      const float ws = share(sd, pz, px);
-      if (ws != 0.f) {
-        const float c = __ldg(a.vp + (long long)pz * a.pitch + px);
-        const float lam = c * a.lamf, mu = c * c * a.muf;
-        acc += ws * ((lam + 2.f * mu) * s_l1[rr - sz][cxm - sx] - lam * s_l2[rr - sz][cxm - sx]);
+      {
+        const float ws = at(w0, w1, i - 1), c = at(c0, c1, i - 1), lam = c * a.lamf, mu = c * c * a.muf;
+        t += ws * ((lam + 2.f * mu) * s_l1[rr][cx + m - SX] - lam * s_l2[rr][cx + m - SX]);
       }
-    }
-    if (dq >= 2) {
-      const int pz = z - 2 * sz, px = xm - 2 * sx;
-      const float ws = share(sd, pz, px);
-      if (ws != 0.f) {
-        const float c = __ldg(a.vp + (long long)pz * a.pitch + px);
-        acc -= ws * c * c * a.muf * s_l1[rr - 2 * sz][cxm - 2 * sx];
+      if (dq <= hw) {  // the depth hw-1 cell's second neighbour is the edge cell instead
+        const float ws = at(w0, w1, i - 2), c = at(c0, c1, i - 2);
+        t -= ws * c * c * a.muf * s_l1[rr][cx + m - 2 * SX];
       }
-    }
-    if (dq == 0) {
-      const int pz = z + (hw - 1) * sz, px = xm + (hw - 1) * sx;
-      if (pz >= 0 && pz < a.nz && px >= 0 && px < a.nx) {
-        const float ws = share(sd, pz, px);
-        if (ws != 0.f) {
-          const long long oo = (long long)pz * a.pitch + px;
+      if (dq == 0) {
+        const int px = xm + (hw - 1) * SX;
+        if (px >= 0 && px < a.nx) {
+          const float ws = share(sd, z, px);
+          const long long oo = (long long)z * a.pitch + px;
           const float c = __ldg(a.vp + oo);
-          acc -= ws * c * c * a.muf * ldf(l1 + oo);
+          if (ws != 0.f) t -= ws * c * c * a.muf * l1[oo];
         }
       }
+      if (xm < a.nx) set_comp(acc, m, comp(acc, m) + t);
     }
-    return acc;
   };
   // top / bottom sides: the four cells share their depth dq, so the strip
   // cells p = q, q - d, q - 2d (and the wrap) are rows of four
@@ -661,34 +706,28 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a) {
       if (pz >= 0 && pz < a.nz) {
         const float4 ws = share4(sd, pz);
         coefs(pz, lam, mu);
-        const float4 lw = ldf4(l1 + (long long)pz * a.pitch + x);
+        const float4 lw = ld4(l1 + (long long)pz * a.pitch + x);
 #pragma unroll
         for (int m = 0; m < 4; ++m) set_comp(acc, m, comp(acc, m) - comp(ws, m) * comp(mu, m) * comp(lw, m));
       }
     }
   };
-  // the one-way sums of the four cells: rows of four for the top and bottom
-  // sides; cell by cell (one rolled copy of the code) for the left and right
-  // sides, in the lanes within their reach only
+  // the one-way sums of the four cells, in the rows and lanes within reach of each side
   float4 ow4 = make_float4(0.f, 0.f, 0.f, 0.f);
   if constexpr (NEAR) {
     if (!mult && z <= hw) oneway_rows(0, z, 1, ow4);
     if (a.nz - 1 - z <= hw) oneway_rows(1, a.nz - 1 - z, -1, ow4);
-    if (x <= hw || x + 3 >= a.nx - 1 - hw) {
-#pragma unroll 1
-      for (int t = 0; t < 8; ++t) {
-        const int m = t >> 1, sd = 2 + (t & 1);
-        const int xm = x + m;
-        if (xm >= a.nx) continue;
-        const int dq = sd == 2 ? xm : a.nx - 1 - xm;
-        if (dq > hw) continue;
-        set_comp(ow4, m, comp(ow4, m) + oneway(sd, dq, 0, sd == 2 ? 1 : -1, xm, cx + m));
-      }
-    }
+    if (x <= hw) oneway_cols(std::integral_constant<int, 1>{}, ow4);
+    if (x + 3 >= a.nx - 1 - hw) oneway_cols(std::integral_constant<int, -1>{}, ow4);
   }
   const float4 wq4 = wi4_at(z, x);
   const float ch = 0.5f * a.w.c[0];
   float v[4], L[4], Lz[4];
+  float4 LK = f0, LU = f0;  // plain equation: L(k wi La1) and L(U_{j-1}) of the four cells
+  if constexpr (!RHO && !VTI) {
+    LK = lap_rows4<R, W>(s_kl, rr, cx, a.w);
+    LU = lap_rows4<R, W>(s_u, rr, cx, a.w);
+  }
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
     const int xm = x + m;
@@ -721,13 +760,8 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a) {
       lu = ux;
       luz = uz;
     } else {
-      lap = a.w.c[0] * s_kl[rr][cx + m];
-      lu = a.w.c[0] * s_u[rr][cx + m];
-#pragma unroll
-      for (int j = 1; j <= R; ++j) {
-        lap += a.w.c[j] * (s_kl[rr - j][cx + m] + s_kl[rr + j][cx + m] + s_kl[rr][cx + m - j] + s_kl[rr][cx + m + j]);
-        lu += a.w.c[j] * (s_u[rr - j][cx + m] + s_u[rr + j][cx + m] + s_u[rr][cx + m - j] + s_u[rr][cx + m + j]);
-      }
+      lap = comp(LK, m);
+      lu = comp(LU, m);
     }
     v[m] = (xm < a.nx) ? 2.f * wq * comp(l1c, m) + lap - wq * comp(l2v, m) + ow : 0.f;
     L[m] = lu;
@@ -850,11 +884,11 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a) {
   if (a.uout != nullptr) *reinterpret_cast<float4*>(a.uout + fb + o) = make_float4(uo[0], uo[1], uo[2], uo[3]);
 }
 
-// The plain / Born equation's kernel is left to the compiler's register
-// choice; the VTI and variable-density ones are held to the CTAs per SM
-// (eight warps each) that their registers allowed before the tile index
-// came from the far block or the frame: near tiles four (variable density
-// two), far tiles three (VTI of order 6 and 8 two).
+// The plain / Born equation's far kernel is left to the compiler's register
+// choice; the others are held to a number of CTAs per SM (eight warps each):
+// near tiles four (variable density two; the plain near kernel at the 80
+// registers the compiler would take fits three: 179 us a step against 148 on 64
+// shots of 500 x 1100), far tiles three (VTI of order 6 and 8 two).
 template <int R, int EQ, bool NEAR>
 constexpr int habc_bwd_min_blocks() {
   if (NEAR) return EQ == 2 ? 2 : 4;
@@ -871,7 +905,18 @@ template <int R, int EQ, bool NEAR>
 __device__ __forceinline__ void habc_bwd_step(const HabcBwdArgs& a) {
   if (!NEAR || a.fx1 <= a.fx0) pdl_wait();
   pdl_trigger();
-  habc_bwd_tile<R, EQ, NEAR>(a);
+  // Far tiles: the resident CTAs walk them (a CTA per tile paid its launch and the
+  // wait above 21504 times a step on 64 shots of 500 x 1100: 141 us, walked 120).
+  // Near tiles: a CTA each (148 us; walked, the loop's registers cost more, 155).
+  if constexpr (NEAR) {
+    habc_bwd_tile<R, EQ, NEAR>(a, blockIdx.x);
+  } else {
+    const int n = a.nfar * a.nshots;
+    for (int t = blockIdx.x; t < n; t += gridDim.x) {
+      if (t != (int)blockIdx.x) __syncthreads();  // the shared tile of the one before is read
+      habc_bwd_tile<R, EQ, NEAR>(a, t);
+    }
+  }
   if (NEAR) pdl_wait();
 }
 template <int R, int EQ, bool NEAR>
@@ -908,6 +953,21 @@ cudaError_t launch_habc_shares(const sgb_grid& g, const sgb_acoustic_model& m, f
   if (blocks > 152 * 8) blocks = 152 * 8;
   habc_shares_kernel<<<(unsigned)blocks, 256, 0, s>>>(g.nz, g.nx, g.pitch, m.habc_width, m.multiple, m.damp, planes);
   return cudaGetLastError();
+}
+
+// A CTA per tile, or (walk) as many as are resident.
+template <auto KERN>
+static cudaError_t launch_tiles(int tiles, bool walk, cudaStream_t s, const HabcBwdArgs& a) {
+  if (!walk) return launch_pdl(KERN, dim3((unsigned)tiles), dim3(32, HT_Z), 0, s, a);
+  static int cap = 0;
+  if (cap == 0) {
+    int nb = 0, dev = 0, sms = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, KERN, 32 * HT_Z, 0) != cudaSuccess || nb < 1) nb = 1;
+    cap = nb * sms;
+  }
+  return launch_pdl(KERN, dim3((unsigned)(tiles < cap ? tiles : cap)), dim3(32, HT_Z), 0, s, a);
 }
 
 cudaError_t launch_habc_bwd(const sgb_grid& g, const sgb_acoustic_model& m, const sgb_acquisition& q,
@@ -986,20 +1046,21 @@ cudaError_t launch_habc_bwd(const sgb_grid& g, const sgb_acoustic_model& m, cons
     a.fz0 = a.fz1 = a.nzb;
     a.fx0 = a.fx1 = 0;
   }
-  const int nfar = (a.fx1 - a.fx0) * (a.fz1 - a.fz0), nnear = a.ntx * a.nzb - nfar;
-  const dim3 gfar((unsigned)(a.fx1 - a.fx0), (unsigned)(a.fz1 - a.fz0), (unsigned)g.nshots);
-  const dim3 gnear((unsigned)nnear, 1u, (unsigned)g.nshots);
+  a.nfar = (a.fx1 - a.fx0) * (a.fz1 - a.fz0);
+  a.nnear = a.ntx * a.nzb - a.nfar;
+  const int nfar = a.nfar, nnear = a.nnear;
   // one launch for the tiles out of reach of the strips, one for the rest
   cudaError_t err = cudaSuccess;
   switch (R * 3 + eq) {
-#define SGB_TILE2(RR, EQ)                                                                           \
-  if constexpr (EQ == 0) {                                                                        \
-    if (nfar > 0 && err == cudaSuccess) err = launch_pdl(habc_bwd_tile_kernel<RR, EQ, false>, gfar, dim3(32, HT_Z), 0, s, a);         \
-    if (nnear > 0 && err == cudaSuccess) err = launch_pdl(habc_bwd_tile_kernel<RR, EQ, true>, gnear, dim3(32, HT_Z), 0, s, a);        \
-  } else {                                                                                        \
-    if (nfar > 0 && err == cudaSuccess) err = launch_pdl(habc_bwd_tile_kernel_held<RR, EQ, false>, gfar, dim3(32, HT_Z), 0, s, a);    \
-    if (nnear > 0 && err == cudaSuccess) err = launch_pdl(habc_bwd_tile_kernel_held<RR, EQ, true>, gnear, dim3(32, HT_Z), 0, s, a);   \
-  }
+#define SGB_TILE2(RR, EQ)                                                                            \
+  if (nfar > 0) {                                                                                    \
+    if constexpr (EQ == 0)                                                                           \
+      err = launch_tiles<habc_bwd_tile_kernel<RR, EQ, false>>(nfar * g.nshots, true, s, a);          \
+    else                                                                                             \
+      err = launch_tiles<habc_bwd_tile_kernel_held<RR, EQ, false>>(nfar * g.nshots, true, s, a);     \
+  }                                                                                                  \
+  if (nnear > 0 && err == cudaSuccess)                                                               \
+    err = launch_tiles<habc_bwd_tile_kernel_held<RR, EQ, true>>(nnear * g.nshots, false, s, a);
     case 3: SGB_TILE2(1, 0) break;
     case 4: SGB_TILE2(1, 1) break;
     case 5: SGB_TILE2(1, 2) break;

@@ -168,6 +168,14 @@ int set_cuda_error(cudaError_t e);
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
+// A pointer whose loads can neither move above this point nor be taken for
+// read-only ones; after pdl_wait, plain loads through it are free to be scheduled
+// (ldf / ldf4 keep their order).
+__device__ __forceinline__ const float* after_wait(const float* p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float ldf(const float* p) {
   float v;
   asm volatile("ld.global.f32 %0, [%1];\n" : "=f"(v) : "l"(p));
