@@ -72,7 +72,7 @@ struct AcVjpArgs {
 // Streaming forward step (PML): TMA-fed per-warp strips.
 struct AcStreamArgs {
   int nz, nx, pitch, nshots, ntx, zc, nzc;
-  int nseg, tpu;  // tiles per column band and per unit (1: every tile stands alone)
+  int variant;  // host: the compiled variant of the launch (fwd_variant)
   const float* __restrict__ um;   // U_{n-1}
   const float* __restrict__ g;    // coefficient planes
   const float* __restrict__ k;
@@ -130,7 +130,6 @@ struct AcFwdBatch {
 // as nu = k * Lambda.
 struct AcBwdStreamArgs {
   int nz, nx, pitch, nshots, ntx, zc, nzc;
-  int nseg, tpu;
   const float* __restrict__ unext;  // U_j
   const float* __restrict__ n2;     // nu_{j+2}
   const float* __restrict__ g;

@@ -78,16 +78,22 @@ __global__ void __launch_bounds__(32 * NWP, TZ / NWP <= 2 ? (PTM >= 2 ? 3 : 4) :
     s_abort = 0;
   }
   for (int i = tid; i < Lay::PF / 4; i += 32 * NWP) sts4(sinj + 4 * i, make_float4(0.f, 0.f, 0.f, 0.f));
-  pdl_wait();
-  pdl_trigger();
-  if (tid == 0)
-    for (int s = 0; s < S; ++s)
-      if ((int)blockIdx.x + s * G < ntiles) issue(s);
-  // the saved ring of U_{j-2}, each CTA a share while its first boxes load:
-  // the tiles never write ring cells, and nothing in this launch reads U_{j-2}
-  if (a.do_recon && a.ring_in != nullptr)
-    ring_copy_share(a.ring, a.nshots, a.pitch, a.sstride, a.uout, const_cast<float*>(a.ring_in), true);
+  // Starts the copies once the step before has ended: called by the first tile
+  // after it has loaded what that step does not write (coefficient rows, sources,
+  // receiver tables and residuals), which so overlaps the step's tail.
+  auto start = [&]() {
+    pdl_wait();
+    pdl_trigger();
+    if (tid == 0)
+      for (int s = 0; s < S; ++s)
+        if ((int)blockIdx.x + s * G < ntiles) issue(s);
+    // the saved ring of U_{j-2}, each CTA a share while its first boxes load:
+    // the tiles never write ring cells, and nothing in this launch reads U_{j-2}
+    if (a.do_recon && a.ring_in != nullptr)
+      ring_copy_share(a.ring, a.nshots, a.pitch, a.sstride, a.uout, const_cast<float*>(a.ring_in), true);
+  };
   __syncthreads();
+  if (PTM == 0) start();  // its point operands are loaded by the warps
   int k = 0;
   for (int t = blockIdx.x; t < ntiles; t += G, ++k, walk.next(TZ)) {
     const int stage = k % S;
@@ -136,6 +142,7 @@ __global__ void __launch_bounds__(32 * NWP, TZ / NWP <= 2 ? (PTM >= 2 ? 3 : 4) :
                               });
       __syncthreads();
     }
+    if (PTM != 0 && k == 0) start();
     if (!mbar_wait(&bars[stage], (k / S) & 1, a.status)) s_abort = 1;
     const float* st = smem + stage * Lay::STAGE;
     const float* sn = st + Lay::UF;

@@ -204,13 +204,21 @@ __device__ __forceinline__ void fwd_tiles(const P& prov, const Pre& pre = Pre{})
     fence_mbar_init();
     s_abort = 0;
   }
-  pdl_wait();
-  pdl_trigger();
-  if (tid == 0)
-    for (int s = 0; s < S; ++s)
-      if ((int)blockIdx.x + s * G < ntiles) issue(blockIdx.x + s * G, s);
-  pre();
+  // Starts the copies once the step before has ended: called by the first tile
+  // after it has loaded what that step does not write (coefficient rows, source
+  // rows, receiver tables), which so overlaps the step's tail.  Operands that the
+  // warps load from the fields come after it (PT false, the HABC additive field).
+  constexpr bool EARLY = PT && HB != 1;
+  auto start = [&]() {
+    pdl_wait();
+    pdl_trigger();
+    if (tid == 0)
+      for (int s = 0; s < S; ++s)
+        if ((int)blockIdx.x + s * G < ntiles) issue(blockIdx.x + s * G, s);
+    pre();
+  };
   __syncthreads();
+  if (!EARLY) start();
   int k = 0;
   for (int t = blockIdx.x; t < ntiles; t += G, ++k) {
     const int stage = k % S;
@@ -276,6 +284,8 @@ __device__ __forceinline__ void fwd_tiles(const P& prov, const Pre& pre = Pre{})
         if (zr.x < g.z0 + TZ && zr.y > g.z0) rec_shots |= 1u << sb;
       }
     }
+    if (rec_shots != 0) prefetch_receivers<TZ, NWP>(a.rec_row_ptr + (long long)b0 * a.nz, a.rec_x, a.rec_col, lane, wid, g.z0, a.nz);
+    if (EARLY && k == 0) start();
     if (!mbar_wait(&bars[stage], (k / S) & 1, a.status)) s_abort = 1;
     const float* st = smem + stage * Lay::STAGE;
     const int lr0 = wid * RPW;
@@ -490,7 +500,7 @@ static cudaError_t fwd_tile_t(const AcFwdBatch<MAXG>& b, cudaStream_t s, bool pr
 
 template <int R, int MAXG>
 static cudaError_t fwd_tile_r(const AcFwdBatch<MAXG>& b, cudaStream_t s, bool prep) {
-  switch (g_fwd_cfg) {
+  switch (b.g[0].variant) {
     case 0: return fwd_tile_t<R, 16, 4, 3, false>(b, s, prep);
     case 1: return fwd_tile_t<R, 16, 4, 3, true>(b, s, prep);
     case 2: return fwd_tile_t<R, 8, 4, 4, true>(b, s, prep);
@@ -512,7 +522,16 @@ static cudaError_t fwd_dispatch(int R, const AcFwdBatch<MAXG>& b, cudaStream_t s
   return cudaErrorInvalidValue;
 }
 
-int fwd_tile_rows() { return FWD_TILE_CFGS[g_fwd_cfg].tz; }
+// The selected variant; in place of the default (16-row tiles, best from two
+// waves of CTAs on) 8-row tiles for grids below that, where a step is the
+// latency of a tile: 4.6 against 5.6 us on 8 shots of 228 x 356 (360 tiles of 16
+// rows), 6.9 against 7.2 on 8 of 356 x 612 (920), but 19.5 against 16.0 on 32 of
+// them (3680).  nshots = 0: a batch of grids, which keeps the selected variant.
+int fwd_variant(int nshots, int nz, int nx) {
+  const long long tiles = (long long)nshots * ((nx + TX - 1) / TX) * ((nz + 15) / 16);
+  return g_fwd_cfg == 4 && nshots > 0 && tiles <= 2 * 608 ? 5 : g_fwd_cfg;
+}
+int fwd_tile_rows(int variant) { return FWD_TILE_CFGS[variant].tz; }
 int fwd_tile_shots() { return FWD_TILE_CFGS[g_fwd_cfg].sb; }
 int stencil_box_width(int R) { return (R % 2 == 0) ? TX + 8 : TX + 16; }
 
@@ -569,6 +588,7 @@ cudaError_t launch_acoustic_fwd_batch(int R, const AcFwdBatch<MAX_BATCH_GROUPS>&
 cudaError_t prepare_acoustic_fwd_batch(int R) {
   AcFwdBatch<MAX_BATCH_GROUPS> b;
   b.ngroups = 0;
+  b.g[0].variant = g_fwd_cfg;
   b.tile0[0] = 0;
   return fwd_dispatch<MAX_BATCH_GROUPS>(R, b, nullptr, true);
 }

@@ -87,7 +87,8 @@ int field_map(CUtensorMap* m, const float* p, int nz, int nx, int pitch, int nsh
               int bs = 1);
 int coef_map(CUtensorMap* m, const float* coef, int nz, int nx, int pitch, int rb);
 int plane_map(CUtensorMap* m, const float* p, int nz, int nx, int pitch, int boxw, int rb);
-int fwd_tile_rows();
+int fwd_variant(int nshots, int nz, int nx);
+int fwd_tile_rows(int variant);
 int fwd_tile_shots();
 int bwd_tile_rows();
 int stencil_box_width(int R);
@@ -190,8 +191,6 @@ void fill_stream_args(AcStreamArgs& sa, const AcStepArgs& a, const sgb_acquisiti
   sa.nz = a.nz; sa.nx = a.nx; sa.pitch = a.pitch; sa.nshots = a.nshots; sa.ntx = a.ntx;
   sa.zc = tzr;
   sa.nzc = (a.nz + tzr - 1) / tzr;
-  sa.nseg = sa.nzc;
-  sa.tpu = 1;
   sa.g = a.g;
   sa.k = a.k;
   sa.src_zr = acq->src_zr;
@@ -496,7 +495,8 @@ int acoustic_forward_impl(const sgb_grid* grid, const sgb_acoustic_model* model,
   CUtensorMap mu[3], mum[3];
   AcStreamArgs sa;
   std::memset(&sa, 0, sizeof(sa));
-  const int tzr = habc ? habc_tile_rows(R, a.rho_c != nullptr ? 3 : (a.kz != nullptr ? 2 : 1)) : fwd_tile_rows();
+  sa.variant = fwd_variant(grid->nshots, grid->nz, grid->nx);
+  const int tzr = habc ? habc_tile_rows(R, a.rho_c != nullptr ? 3 : (a.kz != nullptr ? 2 : 1)) : fwd_tile_rows(sa.variant);
   const int tsb = habc ? 1 : fwd_tile_shots();
   const int bw = stencil_box_width(R);
   for (int i = 0; i < 3; ++i)
@@ -879,8 +879,6 @@ int acoustic_backward_impl(const sgb_grid* grid, const sgb_acoustic_model* model
   sb.ntx = (grid->nx + TX - 1) / TX;
   sb.zc = tzr;
   sb.nzc = (grid->nz + tzr - 1) / tzr;
-  sb.nseg = sb.nzc;
-  sb.tpu = 1;
   sb.g = model->coef;
   sb.k = model->coef + plane;
   sb.src_zr = acq->src_zr;

@@ -13,7 +13,8 @@ namespace sgb {
 FdWeights fd_weights(int order);
 int field_map(CUtensorMap* m, const float* p, int nz, int nx, int pitch, int nshots, int boxw, int rb,
               int bs = 1);
-int fwd_tile_rows();
+int fwd_variant(int nshots, int nz, int nx);
+int fwd_tile_rows(int variant);
 int stencil_box_width(int R);
 cudaError_t launch_acoustic_fwd_batch(int R, const AcFwdBatch<MAX_BATCH_GROUPS>& b, cudaStream_t s);
 cudaError_t prepare_acoustic_fwd_batch(int R);
@@ -62,8 +63,6 @@ AcStreamArgs group_args(const sgb_batch_group& G, int tzr) {
   a.ntx = (g.nx + TX - 1) / TX;
   a.zc = tzr;
   a.nzc = (g.nz + tzr - 1) / tzr;
-  a.nseg = a.nzc;
-  a.tpu = 1;
   const long long plane = (long long)g.nz * g.pitch;
   a.g = G.model.coef;
   a.k = G.model.coef + plane;
@@ -96,7 +95,8 @@ int run_batch(const sgb_batch_group* groups, int ng, int32_t* cur_out, int32_t* 
   for (int g = 0; g < ng; ++g)
     if (int e = check_group(groups[g], order)) return e;
   const int R = order / 2;
-  const int tzr = fwd_tile_rows();
+  const int variant = fwd_variant(0, 0, 0);  // one for the batch: the selected one
+  const int tzr = fwd_tile_rows(variant);
   const int bw = stencil_box_width(R);
   std::vector<GroupMaps> maps(ng);
   std::vector<AcStreamArgs> args(ng);
@@ -109,6 +109,7 @@ int run_batch(const sgb_batch_group* groups, int ng, int32_t* cur_out, int32_t* 
           field_map(&maps[g].point[i], G.buf[i], G.grid.nz, G.grid.nx, G.grid.pitch, G.grid.nshots, TX, tzr))
         return SGB_ERR_CUDA;
     args[g] = group_args(G, tzr);
+    args[g].variant = variant;
     nt_max = G.acq.nt > nt_max ? G.acq.nt : nt_max;
   }
   if (zero) {

@@ -189,6 +189,19 @@ __device__ __forceinline__ void tile_receivers(const int* rp, const int* rec_x, 
   }
 }
 
+// Brings the table entries that tile_receivers will read first into L1, issued
+// before a stage wait so that only the sampling itself follows the tile's stores.
+template <int TZ, int NWP>
+__device__ __forceinline__ void prefetch_receivers(const int* rp, const int* rec_x, const int* rec_col, int lane,
+                                                   int wid, int z0, int nz) {
+  const int p0 = __ldg(rp + z0), p1 = __ldg(rp + min(z0 + TZ, nz));
+  const int q = p0 + (wid * 32 + lane) * 8;  // 32 bytes of each table per thread
+  if (q < p1) {
+    asm volatile("prefetch.global.L1 [%0];\n" ::"l"(rec_x + q));
+    asm volatile("prefetch.global.L1 [%0];\n" ::"l"(rec_col + q));
+  }
+}
+
 // This CTA's share of a boundary-ring copy between a field
 // [nshots][nz][pitch] and its slots [nshots][ring.size] (slot order of
 // Ring::index): scatter = slots -> field, else field -> slots.  Four
