@@ -52,23 +52,27 @@ __device__ __forceinline__ float4 blend4(const float4& y, const float4& U0, cons
 // Which single side every cell of the group x..x+3 in row z takes, under the
 // mask precedence and corner diagonals of acoustic_habc.py:167-202 (cells of
 // no side have b = 0): 0 top, 1 bottom, 2 left, 3 right, or -1 when the
-// group holds a corner, a diagonal or cells of two sides.
+// group holds a diagonal, cells of two sides or cells beyond the grid.
 __device__ __forceinline__ int group_side(int z, int x, int nz, int nx, int hw, bool mult) {
+  if (x + 3 >= nx) return -1;
   const int dB = nz - 1 - z;
-  if ((z >= hw || mult) && dB >= hw) {      // rows without a top or bottom strip
+  const bool top = !mult && z < hw, bot = dB < hw;
+  if (!top && !bot) {  // rows without a top or bottom strip
     if (x + 3 < nx - hw) return 2;
     if (x >= hw) return 3;
     return -1;
   }
-  if (!mult && z < hw && dB >= hw) {
-    const int xd = nx - hw + z;              // top-right diagonal
-    if (x > z && x + 3 < nx - 1 - z && !(xd >= x && xd <= x + 3)) return 0;
-    return -1;
-  }
-  if (dB < hw && z >= hw) {
-    const int xd = hw - 1 - dB;              // bottom-left diagonal
-    if (x > dB && x + 3 < nx - 1 - dB && !(xd >= x && xd <= x + 3)) return 1;
-  }
+  if (bot && z < hw) return -1;
+  // d rows from the strip's edge: left of both diagonals the left side wins,
+  // right of them the right one (each tested against both, for grids narrower
+  // than two strips); the second diagonal of the row (top-right, bottom-left)
+  // follows the block, not the geometry
+  const int d = top ? z : dB;
+  const int xd = top ? nx - hw + z : hw - 1 - dB;
+  if (xd >= x && xd <= x + 3) return -1;
+  if (x > d && x + 3 < nx - 1 - d) return top ? 0 : 1;
+  if (x + 3 < d && x + 3 < nx - 1 - d) return 2;
+  if (x > nx - 1 - d && x > d) return 3;
   return -1;
 }
 
@@ -97,18 +101,15 @@ __device__ __forceinline__ void lap_row_xz(const float4 (&win)[2 * R + 1], const
 
 // PT: the previous field travels through the TMA stage (prefetched S-1
 // tiles ahead) instead of a global load issued before the stage wait.
-// SB: shots per tile; one TMA box carries all SB shots (shot is the box's
-// third dimension), the coefficient rows and the tile's barrier are shared.
-template <int R, int TZ, int S, bool PT, int SB = 1>
+template <int R, int TZ, int S, bool PT>
 struct FwdTileLayout {
   static constexpr int UW = Row<R>::W;
   static constexpr int UROWS = TZ + 2 * R;
-  static constexpr int USHOT = UROWS * UW;  // floats of one shot's stencil box
-  static constexpr int UF = round32(SB * USHOT);
-  static constexpr int PSHOT = TZ * TX;
-  static constexpr int STAGE = UF + (PT ? SB * PSHOT : 0);
+  static constexpr int UF = round32(UROWS * UW);
+  static constexpr int PF = TZ * TX;
+  static constexpr int STAGE = UF + (PT ? PF : 0);
   static constexpr size_t BYTES = (size_t)S * STAGE * 4 + S * 8;
-  static constexpr uint32_t TX_BYTES = (SB * USHOT + (PT ? SB * PSHOT : 0)) * 4;
+  static constexpr uint32_t TX_BYTES = (UROWS * UW + (PT ? PF : 0)) * 4;
 };
 
 // Tile providers: the single-grid kernel takes its tensor maps and argument
@@ -116,20 +117,15 @@ struct FwdTileLayout {
 // bank); the batch kernel covers every tile of up to MAXG grids (an uneven
 // batch: each group has its own shape, shots, buffers and step), tiles
 // numbered group after group from tile0[g].
-template <int SB>
 struct FwdOne {
-  static constexpr bool ONE = true;
+  static constexpr bool WALK = true;
   using Walk = TileWalk;
-  template <int>
-  __device__ __forceinline__ Walk walk(int t, int G, int tz) const {
-    return TileWalk(t, G, (a.nshots + SB - 1) / SB, a.ntx, tz);
-  }
   const CUtensorMap* tu;
   const CUtensorMap* tum;
   AcStreamArgs a;
-  __device__ __forceinline__ int ntiles() const { return (a.nshots + SB - 1) / SB * a.ntx * a.nzc; }
+  __device__ __forceinline__ int ntiles() const { return a.nshots * a.ntx * a.nzc; }
+  __device__ __forceinline__ Walk walk(int t, int G, int tz) const { return TileWalk(t, G, a.nshots, a.ntx, tz); }
   __device__ __forceinline__ int group(int) const { return 0; }
-  __device__ __forceinline__ int first(int) const { return 0; }
   __device__ __forceinline__ const AcStreamArgs& args(int) const { return a; }
   __device__ __forceinline__ const CUtensorMap* map_u(int) const { return tu; }
   __device__ __forceinline__ const CUtensorMap* map_um(int) const { return tum; }
@@ -137,18 +133,19 @@ struct FwdOne {
 
 template <int MAXG>
 struct FwdMany {
-  static constexpr bool ONE = false;
+  static constexpr bool WALK = false;
   struct Walk {};
-  template <int>
-  __device__ __forceinline__ Walk walk(int, int, int) const { return {}; }
   const AcFwdBatch<MAXG>& B;
   __device__ __forceinline__ int ntiles() const { return B.tile0[B.ngroups]; }
+  __device__ __forceinline__ Walk walk(int, int, int) const { return {}; }
+  __device__ __forceinline__ Tile geom(int t, int gi, int tz) const {
+    return tile_geom(t - B.tile0[gi], B.g[gi].nshots, B.g[gi].ntx, tz);
+  }
   __device__ __forceinline__ int group(int t) const {
     int gi = 0;
     while (gi + 1 < B.ngroups && t >= B.tile0[gi + 1]) ++gi;
     return gi;
   }
-  __device__ __forceinline__ int first(int gi) const { return B.tile0[gi]; }
   __device__ __forceinline__ const AcStreamArgs& args(int gi) const { return B.g[gi]; }
   __device__ __forceinline__ const CUtensorMap* map_u(int gi) const { return &B.tm_u[gi]; }
   __device__ __forceinline__ const CUtensorMap* map_um(int gi) const { return &B.tm_um[gi]; }
@@ -164,11 +161,9 @@ struct FwdMany {
 struct NoPre {
   __device__ __forceinline__ void operator()() const {}
 };
-template <int R, int TZ, int NWP, int S, bool PT, int SB, class P, int HB = 0, class Pre = NoPre>
+template <int R, int TZ, int NWP, int S, bool PT, class P, int HB = 0, class Pre = NoPre>
 __device__ __forceinline__ void fwd_tiles(const P& prov, const Pre& pre = Pre{}) {
-  static_assert(SB == 1 || PT, "several shots per tile need the previous field in the stage");
-  static_assert(HB == 0 || SB == 1, "the HABC family runs one shot per tile (its rows are read for shot b0)");
-  using Lay = FwdTileLayout<R, TZ, S, PT, SB>;
+  using Lay = FwdTileLayout<R, TZ, S, PT>;
   constexpr int RPW = TZ / NWP;
   constexpr int UW = Lay::UW, LO = Row<R>::LO;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -180,24 +175,24 @@ __device__ __forceinline__ void fwd_tiles(const P& prov, const Pre& pre = Pre{})
   const int G = gridDim.x;
 
   // tile geometry: a walk without divisions on one grid, per tile over several
-  typename P::Walk walk = prov.template walk<SB>(blockIdx.x, G, TZ), ahead = walk;  // this tile, the next one to load
-  auto geom = [&](typename P::Walk& w, int t, int gi, const AcStreamArgs& a) -> Tile {
-    if constexpr (P::ONE) {
+  typename P::Walk walk = prov.walk(blockIdx.x, G, TZ), ahead = walk;  // this tile, the next one to load
+  auto geom = [&](typename P::Walk& w, int t, int gi) -> Tile {
+    if constexpr (P::WALK) {
       const Tile g = w.g;
       w.next(TZ);
       return g;
     } else {
-      return tile_geom(t - prov.first(gi), (a.nshots + SB - 1) / SB, a.ntx, TZ);
+      return prov.geom(t, gi, TZ);
     }
   };
   auto issue = [&](int t, int stage) {
     const int gi = prov.group(t);
-    const Tile g = geom(ahead, t, gi, prov.args(gi));
+    const Tile g = geom(ahead, t, gi);
     fence_proxy_async_smem();
     mbar_arrive_expect_tx(&bars[stage], Lay::TX_BYTES);
-    tma_load_3d(smem + stage * Lay::STAGE, prov.map_u(gi), g.x0 - LO, g.z0 - R, g.b * SB, &bars[stage]);
+    tma_load_3d(smem + stage * Lay::STAGE, prov.map_u(gi), g.x0 - LO, g.z0 - R, g.b, &bars[stage]);
     if (PT)
-      tma_load_3d(smem + stage * Lay::STAGE + Lay::UF, prov.map_um(gi), g.x0, g.z0, g.b * SB, &bars[stage]);
+      tma_load_3d(smem + stage * Lay::STAGE + Lay::UF, prov.map_um(gi), g.x0, g.z0, g.b, &bars[stage]);
   };
   if (tid == 0) {
     for (int s = 0; s < S; ++s) mbar_init(&bars[s], 1);
@@ -224,11 +219,12 @@ __device__ __forceinline__ void fwd_tiles(const P& prov, const Pre& pre = Pre{})
     const int stage = k % S;
     const int gi = prov.group(t);
     const AcStreamArgs& a = prov.args(gi);
-    const Tile g = geom(walk, t, gi, a);
+    const Tile g = geom(walk, t, gi);
     const int x = g.x0 + 4 * lane;
     const bool xin = x < a.nx;
     const int zw = g.z0 + wid * RPW;  // first row of this warp
-    const int b0 = g.b * SB;          // first shot of the tile
+    const int b = g.b;
+    const long long fbase = (long long)b * a.sstride;
     // point operands of this warp's rows, issued before the stage wait (the
     // coefficient rows serve every shot of the tile)
     float4 vm[RPW], vg[RPW], vk[RPW];
@@ -238,13 +234,13 @@ __device__ __forceinline__ void fwd_tiles(const P& prov, const Pre& pre = Pre{})
     // the viscoacoustic term): its rows; else the Born background's m rows
     float4 vbn[HB == 1 ? RPW : 1];
     const float* bnp = nullptr;
-    if constexpr (HB == 1) bnp = a.born_in != nullptr ? a.born_in + (long long)b0 * a.sstride : a.born_m;
+    if constexpr (HB == 1) bnp = a.born_in != nullptr ? a.born_in + fbase : a.born_m;
 #pragma unroll
     for (int i = 0; i < RPW; ++i) {
       const int z = zw + i;
       if (xin && z < a.nz) {
         const long long mo = (long long)z * a.pitch + x;
-        if (!PT) vm[i] = ldf4(a.um + (long long)b0 * a.sstride + mo);
+        if (!PT) vm[i] = ldf4(a.um + fbase + mo);
         vg[i] = ldg4(a.g + mo);
         vk[i] = ldg4(a.k + mo);
         if constexpr (HB == 2) vkz[i] = ldg4(a.kz + mo);
@@ -264,45 +260,33 @@ __device__ __forceinline__ void fwd_tiles(const P& prov, const Pre& pre = Pre{})
         }
       }
     }
-    // source rows of the tile's shots, read before the stage wait as well
-    int2 szr[SB];
-#pragma unroll
-    for (int sb = 0; sb < SB; ++sb) {
-      szr[sb] = make_int2(0, 0);
-      if (a.src_ptr != nullptr && b0 + sb < a.nshots) szr[sb] = __ldg(reinterpret_cast<const int2*>(a.src_zr) + b0 + sb);
-    }
+    // the shot's source rows, read before the stage wait as well
+    int2 szr = make_int2(0, 0);
+    if (a.src_ptr != nullptr) szr = __ldg(reinterpret_cast<const int2*>(a.src_zr) + b);
     // illumination as 16-byte reductions where the plane is 16-byte aligned
     // (four scalar atomics per lane: 43.7 us a step with it on the 32-shot
     // 356 x 612 fourth-order grid)
     const bool illum4 = (reinterpret_cast<uintptr_t>(a.illum) & 15u) == 0;
-    unsigned rec_shots = 0;  // bit sb: shot b0 + sb has receivers in this band
+    bool has_rec = false;  // the shot has receivers in this band
     if (a.records != nullptr) {
-#pragma unroll
-      for (int sb = 0; sb < SB; ++sb) {
-        if (b0 + sb >= a.nshots) break;
-        const int2 zr = __ldg(reinterpret_cast<const int2*>(a.rec_zr) + b0 + sb);
-        if (zr.x < g.z0 + TZ && zr.y > g.z0) rec_shots |= 1u << sb;
-      }
+      const int2 zr = __ldg(reinterpret_cast<const int2*>(a.rec_zr) + b);
+      has_rec = zr.x < g.z0 + TZ && zr.y > g.z0;
     }
-    if (rec_shots != 0) prefetch_receivers<TZ, NWP>(a.rec_row_ptr + (long long)b0 * a.nz, a.rec_x, a.rec_col, lane, wid, g.z0, a.nz);
+    if (has_rec)
+      prefetch_receivers<TZ, NWP>(a.rec_row_ptr + (long long)b * a.nz, a.rec_x, a.rec_col, lane, wid, g.z0, a.nz);
     if (EARLY && k == 0) start();
     if (!mbar_wait(&bars[stage], (k / S) & 1, a.status)) s_abort = 1;
-    const float* st = smem + stage * Lay::STAGE;
+    const float* su = smem + stage * Lay::STAGE;
     const int lr0 = wid * RPW;
+    if (PT) {
 #pragma unroll
-    for (int sb = 0; sb < SB; ++sb) {
-      const int b = b0 + sb;
-      if (b >= a.nshots) break;
-      const long long fbase = (long long)b * a.sstride;
-      const float* su = st + sb * Lay::USHOT;
-      if (PT) {
-#pragma unroll
-        for (int i = 0; i < RPW; ++i) vm[i] = lds4(st + Lay::UF + sb * Lay::PSHOT + (lr0 + i) * TX + 4 * lane);
-      }
-      WarpSrc src{0u, -1, 0, 0.f};
-      if (a.src_ptr != nullptr && szr[sb].x < zw + RPW && szr[sb].y > zw)
-        src = warp_sources(lane, b, zw, RPW, g.x0, a.src_ptr, a.src_z, a.src_x, a.src_wrow, a.wavelet, a.nt, a.t,
-                           a.status);
+      for (int i = 0; i < RPW; ++i) vm[i] = lds4(su + Lay::UF + (lr0 + i) * TX + 4 * lane);
+    }
+    WarpSrc src{0u, -1, 0, 0.f};
+    if (a.src_ptr != nullptr && szr.x < zw + RPW && szr.y > zw)
+      src = warp_sources(lane, b, zw, RPW, g.x0, a.src_ptr, a.src_z, a.src_x, a.src_wrow, a.wavelet, a.nt, a.t,
+                         a.status);
+    {
       float4 win[2 * R + 1];
 #pragma unroll
       for (int j = 0; j < 2 * R; ++j) win[j] = lds4(su + (lr0 + j) * UW + LO + 4 * lane);
@@ -356,11 +340,10 @@ __device__ __forceinline__ void fwd_tiles(const P& prov, const Pre& pre = Pre{})
             }
           }
         }
-        if (HB != 0 && z < a.nz && xin && (z < a.hw || z >= a.nz - a.hw || x < a.hw || x + 3 >= a.nx - a.hw)) {
-          // the one-way blend on strip cells: four cells of one side at once,
-          // else cell by cell (corners, diagonals, mixed groups; one copy of
-          // its code, not unrolled)
-          const int side = (x + 3 < a.nx) ? group_side(z, x, a.nz, a.nx, a.hw, a.multiple != 0) : -1;
+        if constexpr (HB != 0) {
+          // the one-way blend on strip cells: four cells of one side at once
+          const bool strip = z < a.nz && xin && (z < a.hw || z >= a.nz - a.hw || x < a.hw || x + 3 >= a.nx - a.hw);
+          const int side = strip ? group_side(z, x, a.nz, a.nx, a.hw, a.multiple != 0) : -1;
           const long long ro = (long long)z * a.pitch + x;
           if (side >= 0) {
             const float4 cv = ldg4(a.vp + ro), bv = ldg4(a.hb + ro);
@@ -387,11 +370,30 @@ __device__ __forceinline__ void fwd_tiles(const P& prov, const Pre& pre = Pre{})
               P1 = make_float4(ldf(a.um + fbase + ro - 1), vm[i].x, vm[i].y, vm[i].z);
             }
             y = blend4(y, c, U1, U2, vm[i], P1, cv, bv, a.lamf, a.muf);
-          } else {
+          }
+          // the groups with a corner diagonal or cells of two sides, each by four
+          // lanes at a time, a cell per lane: one lane's four cells in turn cost its
+          // warp four times as long.  Every row of a corner has such a group; with
+          // this, and the corner's other groups taken as of one side, 64 shots of
+          // 500 x 1100 take 125 us a step (131 with whole corners cell by cell).
+          // The far tiles in a launch of their own, without this code, were slower:
+          // 51 + 91 us, the frame's tiles alone leave the memory idle.
+          unsigned slow = __ballot_sync(FULL, strip && side < 0);
+          if (slow != 0) {
             const StageField T{su, g.z0 - R, g.x0 - LO, TZ + 2 * R, UW, a.u, a.um, fbase, a.pitch};
 #pragma unroll 1
-            for (int m = 0; m < 4; ++m)
-              if (x + m < a.nx) set_comp(y, m, habc_point(T, a, z, x + m, comp(y, m)));
+            do {
+              const int l = __ffs(slow) - 1;
+              slow &= slow - 1;
+              const int xc = g.x0 + 4 * l + (lane & 3);
+              const float y0 = __shfl_sync(FULL, y.x, l), y1 = __shfl_sync(FULL, y.y, l);
+              const float y2 = __shfl_sync(FULL, y.z, l), y3 = __shfl_sync(FULL, y.w, l);
+              float v = (lane & 2) ? ((lane & 1) ? y3 : y2) : ((lane & 1) ? y1 : y0);
+              if (lane < 4 && xc < a.nx) v = habc_point(T, a, z, xc, v);
+              const float v0 = __shfl_sync(FULL, v, 0), v1 = __shfl_sync(FULL, v, 1);
+              const float v2 = __shfl_sync(FULL, v, 2), v3 = __shfl_sync(FULL, v, 3);
+              if (lane == l) y = make_float4(v0, v1, v2, v3);
+            } while (slow != 0);
           }
         }
         if (src.mask) apply_sources(src, i, lane, 1.f, y);
@@ -416,16 +418,12 @@ __device__ __forceinline__ void fwd_tiles(const P& prov, const Pre& pre = Pre{})
     // stage free; this tile's outputs visible to the CTA; abort is uniform
     if (__syncthreads_or(s_abort)) break;
     if (tid == 0 && t + S * G < ntiles) issue(t + S * G, stage);
-    for (int sb = 0; sb < SB; ++sb) {
-      if (!(rec_shots & (1u << sb))) continue;
-      const int b = b0 + sb;
-      const long long fbase = (long long)b * a.sstride;
+    if (has_rec)
       tile_receivers<TZ, NWP>(a.rec_row_ptr + (long long)b * a.nz, a.rec_x, a.rec_col, lane, wid, g.x0, g.z0, a.nz,
                               [&](int lr, int rx, int col) {
                                 a.records[(long long)col * a.nch] =
                                     a.un[fbase + (long long)(g.z0 + lr) * a.pitch + g.x0 + rx];
                               });
-    }
   }
   // drain: wait (bounded) for the boxes this CTA issued but did not consume
   if (s_abort && tid == 0)
@@ -436,43 +434,41 @@ __device__ __forceinline__ void fwd_tiles(const P& prov, const Pre& pre = Pre{})
 // the second-order HABC instantiations with two rows per warp run 640
 // threads per SM (registers held to 102), the others, and the PML ones, 512
 // (128 registers)
-template <int R, int TZ, int NWP, int S, bool PT, int SB, int HB = 0>
-__global__ void __launch_bounds__(32 * NWP, HB != 0 ? ((R == 1 && TZ / NWP <= 2) ? 20 : 16) / NWP : 16 / NWP)
-    acoustic_fwd_tile_kernel(const __grid_constant__ CUtensorMap tm_u,
-                                                                     const __grid_constant__ CUtensorMap tm_um,
-                                                                     const AcStreamArgs a) {
+template <int R, int TZ, int NWP, int S, bool PT, int HB = 0>
+__global__ void __launch_bounds__(32 * NWP, (HB != 0 && R == 1 && TZ / NWP <= 2 ? 20 : 16) / NWP)
+    acoustic_fwd_tile_kernel(const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ CUtensorMap tm_um,
+                             const AcStreamArgs a) {
   // the input field's boundary ring for the adjoint, each CTA a share while
   // its first boxes load (the input is read-only in this launch)
   auto ring = [&]() {
     if (a.ring_dst != nullptr)
       ring_copy_share(a.ring, a.nshots, a.pitch, a.sstride, const_cast<float*>(a.ring_src), a.ring_dst, false);
   };
-  fwd_tiles<R, TZ, NWP, S, PT, SB, FwdOne<SB>, HB>(FwdOne<SB>{&tm_u, &tm_um, a}, ring);
+  fwd_tiles<R, TZ, NWP, S, PT, FwdOne, HB>(FwdOne{&tm_u, &tm_um, a}, ring);
 }
 
 template <int R, int TZ, int NWP, int S, bool PT, int MAXG>
 __global__ void __launch_bounds__(32 * NWP) acoustic_fwd_batch_kernel(const __grid_constant__ AcFwdBatch<MAXG> B) {
-  fwd_tiles<R, TZ, NWP, S, PT, 1>(FwdMany<MAXG>{B});
+  fwd_tiles<R, TZ, NWP, S, PT>(FwdMany<MAXG>{B});
 }
 
 // ------------------------------------------------------------- launch ---
 
 struct FwdCfg {
-  int tz, nwp, s, sb;
+  int tz, nwp, s;
 };
-static const FwdCfg FWD_TILE_CFGS[] = {{16, 4, 3, 1}, {16, 4, 3, 1}, {8, 4, 4, 1},
-                                       {32, 8, 2, 1}, {16, 4, 2, 1}, {8, 4, 3, 1}};
+static const FwdCfg FWD_TILE_CFGS[] = {{16, 4, 3}, {16, 4, 3}, {8, 4, 4}, {32, 8, 2}, {16, 4, 2}, {8, 4, 3}};
 
 // Launches the variant on batch b; with s == nullptr and prepare_only it
 // only sets the kernel's shared-memory attribute (done once per variant, and
 // before any stream capture).
-template <int R, int TZ, int NWP, int S, bool PT, int MAXG, int SB = 1, int HB = 0>
+template <int R, int TZ, int NWP, int S, bool PT, int MAXG, int HB = 0>
 static cudaError_t fwd_tile_t(const AcFwdBatch<MAXG>& b, cudaStream_t s, bool prepare_only) {
-  using Lay = FwdTileLayout<R, TZ, S, PT, MAXG == 1 ? SB : 1>;
+  using Lay = FwdTileLayout<R, TZ, S, PT>;
   const size_t smem = Lay::BYTES + 128;  // + alignment slack
   static int blocks = 0;
   if constexpr (MAXG == 1) {
-    auto kern = acoustic_fwd_tile_kernel<R, TZ, NWP, S, PT, SB, HB>;
+    auto kern = acoustic_fwd_tile_kernel<R, TZ, NWP, S, PT, HB>;
     if (blocks == 0) {
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
@@ -480,7 +476,7 @@ static cudaError_t fwd_tile_t(const AcFwdBatch<MAXG>& b, cudaStream_t s, bool pr
     }
     if (prepare_only) return cudaSuccess;
     const AcStreamArgs& a = b.g[0];
-    const int tiles = (a.nshots + SB - 1) / SB * a.ntx * a.nzc;
+    const int tiles = a.nshots * a.ntx * a.nzc;
     if (tiles <= 0) return cudaSuccess;
     return launch_pdl(kern, dim3((unsigned)(tiles < blocks ? tiles : blocks)), dim3(32 * NWP), smem, s, b.tm_u[0],
                       b.tm_um[0], b.g[0]);
@@ -501,12 +497,12 @@ static cudaError_t fwd_tile_t(const AcFwdBatch<MAXG>& b, cudaStream_t s, bool pr
 template <int R, int MAXG>
 static cudaError_t fwd_tile_r(const AcFwdBatch<MAXG>& b, cudaStream_t s, bool prep) {
   switch (b.g[0].variant) {
-    case 0: return fwd_tile_t<R, 16, 4, 3, false>(b, s, prep);
-    case 1: return fwd_tile_t<R, 16, 4, 3, true>(b, s, prep);
-    case 2: return fwd_tile_t<R, 8, 4, 4, true>(b, s, prep);
-    case 3: return fwd_tile_t<R, 32, 8, 2, true>(b, s, prep);
-    case 4: return fwd_tile_t<R, 16, 4, 2, true>(b, s, prep);
-    case 5: return fwd_tile_t<R, 8, 4, 3, true>(b, s, prep);
+    case 0: return fwd_tile_t<R, 16, 4, 3, false, MAXG>(b, s, prep);
+    case 1: return fwd_tile_t<R, 16, 4, 3, true, MAXG>(b, s, prep);
+    case 2: return fwd_tile_t<R, 8, 4, 4, true, MAXG>(b, s, prep);
+    case 3: return fwd_tile_t<R, 32, 8, 2, true, MAXG>(b, s, prep);
+    case 4: return fwd_tile_t<R, 16, 4, 2, true, MAXG>(b, s, prep);
+    case 5: return fwd_tile_t<R, 8, 4, 3, true, MAXG>(b, s, prep);
   }
   return cudaErrorInvalidValue;
 }
@@ -532,7 +528,6 @@ int fwd_variant(int nshots, int nz, int nx) {
   return g_fwd_cfg == 4 && nshots > 0 && tiles <= 2 * 608 ? 5 : g_fwd_cfg;
 }
 int fwd_tile_rows(int variant) { return FWD_TILE_CFGS[variant].tz; }
-int fwd_tile_shots() { return FWD_TILE_CFGS[g_fwd_cfg].sb; }
 int stencil_box_width(int R) { return (R % 2 == 0) ? TX + 8 : TX + 16; }
 
 // The HABC family's forward: HT-row tiles, 4 warps, HS stages, previous
@@ -561,22 +556,22 @@ cudaError_t launch_acoustic_fwd_stream(int R, const CUtensorMap* maps, const AcS
   b.tile0[1] = a.nshots * a.ntx * a.nzc;
   if (!habc) return fwd_dispatch<1>(R, b, s, false);
   // variable density and VTI are second order (the reference's kernels)
-  if (a.rho_c != nullptr) return R == 1 ? fwd_tile_t<1, HT, 4, HS, true, 1, 1, 3>(b, s, false) : cudaErrorInvalidValue;
-  if (a.kz != nullptr) return R == 1 ? fwd_tile_t<1, HT, 4, HS, true, 1, 1, 2>(b, s, false) : cudaErrorInvalidValue;
+  if (a.rho_c != nullptr) return R == 1 ? fwd_tile_t<1, HT, 4, HS, true, 1, 3>(b, s, false) : cudaErrorInvalidValue;
+  if (a.kz != nullptr) return R == 1 ? fwd_tile_t<1, HT, 4, HS, true, 1, 2>(b, s, false) : cudaErrorInvalidValue;
   switch (R) {
     case 1:
       switch (g_habc_fwd_cfg) {
-        case 0: return fwd_tile_t<1, 8, 4, 3, true, 1, 1, 1>(b, s, false);
-        case 1: return fwd_tile_t<1, 16, 4, 2, true, 1, 1, 1>(b, s, false);
-        case 2: return fwd_tile_t<1, 16, 4, 3, true, 1, 1, 1>(b, s, false);
-        case 3: return fwd_tile_t<1, 8, 4, 4, false, 1, 1, 1>(b, s, false);
-        case 4: return fwd_tile_t<1, 16, 4, 3, false, 1, 1, 1>(b, s, false);
-        case 5: return fwd_tile_t<1, 32, 8, 2, true, 1, 1, 1>(b, s, false);
+        case 0: return fwd_tile_t<1, 8, 4, 3, true, 1, 1>(b, s, false);
+        case 1: return fwd_tile_t<1, 16, 4, 2, true, 1, 1>(b, s, false);
+        case 2: return fwd_tile_t<1, 16, 4, 3, true, 1, 1>(b, s, false);
+        case 3: return fwd_tile_t<1, 8, 4, 4, false, 1, 1>(b, s, false);
+        case 4: return fwd_tile_t<1, 16, 4, 3, false, 1, 1>(b, s, false);
+        case 5: return fwd_tile_t<1, 32, 8, 2, true, 1, 1>(b, s, false);
       }
       return cudaErrorInvalidValue;
-    case 2: return fwd_tile_t<2, HT, 4, HS, true, 1, 1, 1>(b, s, false);
-    case 3: return fwd_tile_t<3, HT, 4, HS, true, 1, 1, 1>(b, s, false);
-    case 4: return fwd_tile_t<4, HT, 4, HS, true, 1, 1, 1>(b, s, false);
+    case 2: return fwd_tile_t<2, HT, 4, HS, true, 1, 1>(b, s, false);
+    case 3: return fwd_tile_t<3, HT, 4, HS, true, 1, 1>(b, s, false);
+    case 4: return fwd_tile_t<4, HT, 4, HS, true, 1, 1>(b, s, false);
   }
   return cudaErrorInvalidValue;
 }

@@ -89,7 +89,6 @@ int coef_map(CUtensorMap* m, const float* coef, int nz, int nx, int pitch, int r
 int plane_map(CUtensorMap* m, const float* p, int nz, int nx, int pitch, int boxw, int rb);
 int fwd_variant(int nshots, int nz, int nx);
 int fwd_tile_rows(int variant);
-int fwd_tile_shots();
 int bwd_tile_rows();
 int stencil_box_width(int R);
 int set_stream_config(int fwd, int bwd, int habc);
@@ -497,11 +496,10 @@ int acoustic_forward_impl(const sgb_grid* grid, const sgb_acoustic_model* model,
   std::memset(&sa, 0, sizeof(sa));
   sa.variant = fwd_variant(grid->nshots, grid->nz, grid->nx);
   const int tzr = habc ? habc_tile_rows(R, a.rho_c != nullptr ? 3 : (a.kz != nullptr ? 2 : 1)) : fwd_tile_rows(sa.variant);
-  const int tsb = habc ? 1 : fwd_tile_shots();
   const int bw = stencil_box_width(R);
   for (int i = 0; i < 3; ++i)
-    if (field_map(&mu[i], buf[i], grid->nz, grid->nx, grid->pitch, grid->nshots, bw, tzr + 2 * R, tsb) ||
-        field_map(&mum[i], buf[i], grid->nz, grid->nx, grid->pitch, grid->nshots, TX, tzr, tsb))
+    if (field_map(&mu[i], buf[i], grid->nz, grid->nx, grid->pitch, grid->nshots, bw, tzr + 2 * R) ||
+        field_map(&mum[i], buf[i], grid->nz, grid->nx, grid->pitch, grid->nshots, TX, tzr))
       return SGB_ERR_CUDA;
   fill_stream_args(sa, a, acq, tzr);
   sa.illum = illum;
