@@ -376,16 +376,27 @@ __global__ void __launch_bounds__(128) elastic_fwd_kernel(const ElFwdArgs a) {
 
 // Rows a reverse iteration r reads, prefetched one iteration ahead (index in
 // the slot): s0 s1 (v_in in mode 1) s2 s3 a0 a2 a3 a4 of r; s4 a1 of r + 1;
-// in mode 1 the three per-shot gradient rows of r.  The coefficient rows
-// (shared by all shots, L2-resident) are read with early __ldg instead.  In
-// mode 0 (the reverse loop) every shot adds its gradient terms into plane 0
-// of each gradient field with 16-byte reduction atomics: the planes stay in
-// L2, and the step moves 80 instead of 104 B per shot-point of DRAM traffic.
+// in mode 0 the saved ring values of the five fields of s_i in row r (copied
+// by the lanes that hold ring cells only), in mode 1 the three per-shot
+// gradient rows of r.  The coefficient rows (shared by all shots, L2-resident)
+// are read with early __ldg instead.  In mode 0 (the reverse loop) every shot
+// adds its gradient terms into plane 0 of each gradient field with 16-byte
+// reduction atomics: the planes stay in L2, and the step moves 80 instead of
+// 104 B per shot-point of DRAM traffic.
+//
+// What bounds mode 0: latency at 12 warps per SM (168 registers, 61 KB per
+// CTA), DRAM at 56 % of its peak.  Everything that few rows need is kept out of
+// the row's straight code: point corrections are one loop over the staged rows
+// that have any, the ring arrives with the prefetch, and the fields share one
+// offset per row.  32 shots of 400 x 900 take 216 us a step; with the
+// corrections and the ring loads inlined at each of the eleven reads and five
+// stores of a row (the warps then wait for instructions as long as for memory)
+// 292 us.  Held to 128 registers it spills and shared memory still allows three CTAs.
 template <int MODE>
-__host__ __device__ constexpr int bwd_pre_rows() { return MODE == 0 ? 10 : 13; }
+__host__ __device__ constexpr int bwd_pre_rows() { return MODE == 0 ? 15 : 13; }
 
 template <int TZ, int MODE>
-__global__ void __launch_bounds__(128) elastic_bwd_kernel(const ElBwdArgs a) {
+__global__ void __launch_bounds__(128, MODE == 0 ? 3 : 2) elastic_bwd_kernel(const ElBwdArgs a) {
   __shared__ __align__(16) float sbuf_all[4][128];
   constexpr int BWD_PRE_ROWS = bwd_pre_rows<MODE>();
   extern __shared__ __align__(16) float bwd_pre[];  // [4 warps][2 slots][BWD_PRE_ROWS][128]
@@ -404,13 +415,6 @@ __global__ void __launch_bounds__(128) elastic_bwd_kernel(const ElBwdArgs a) {
   const ElLane L = make_lane(x0, a.nx, a.pitch);
   const RowIO io{a.nz, a.pitch};
   const long long fb = (long long)b * a.sstride;
-  const float* S[5];
-  const float* A[5];
-#pragma unroll
-  for (int f = 0; f < 5; ++f) {
-    S[f] = a.s_in[f] + fb;
-    A[f] = a.a_in[f] + fb;
-  }
   // box columns of this lane (mode 1: every column)
   const unsigned boxc = MODE == 0 ? col_mask(L, a.ring.ix0, a.ring.ix1) : 0xFu;
   const WarpPts src = MODE == 0 ? load_sources(a.p, b, z0 - 1, z1 + 2, x0 - 4, x0 + 124, a.status)
@@ -438,57 +442,74 @@ __global__ void __launch_bounds__(128) elastic_bwd_kernel(const ElBwdArgs a) {
     }
     return v;
   };
-  auto lds = [&](int f, int z) { return fix_s(io.ldfield(S[f], z, L), f, z); };
-  auto lda = [&](int f, int z) { return fix_a(io.ldfield(A[f], z, L), f, z); };
-  auto cp_row = [&](float* dst, const float* src, int zz) {
-    const bool ok = L.ld && zz >= 0 && zz < nz;
-    cp_async16(dst + 4 * L.lane, ok ? src + (long long)zz * a.pitch + L.xl : src, ok ? 16 : 0);
+  auto lds = [&](int f, int z) { return fix_s(io.ldfield(a.s_in[f] + fb, z, L), f, z); };
+  auto lda = [&](int f, int z) { return fix_a(io.ldfield(a.a_in[f] + fb, z, L), f, z); };
+  // the same on iteration r's staged rows, in place
+  auto fix_row = [&](float* d, int r) {
+    float* own = d + 4 * L.lane;
+    if (src.any != 0u) {
+#pragma unroll 1
+      for (int f = 0; f < 5; ++f) {
+        float* row = own + (f == 4 ? 8 : f) * 128;
+        sts4(row, fix_s(lds4(row), f, f == 4 ? r + 1 : r));
+      }
+    }
+    if (has_rec) {
+#pragma unroll 1
+      for (int ch = 0; ch < a.p.nch; ++ch) {
+        const int f = a.p.rec_fields[ch];
+        const int z = f == 1 ? r + 1 : r;
+        if (z < 0 || z >= nz) continue;
+        float* row = own + (f == 0 ? 4 : f == 1 ? 9 : f + 3) * 128;
+        float4 v = lds4(row);
+        add_residual(pr, a.resid, z, ch, v, sbuf, L);
+        sts4(row, v);
+      }
+    }
   };
   // v into row z of plane 0 of a gradient field (this lane's four columns)
   auto gred = [&](float* plane, int z, const float4& v) {
     if (L.own) red_add4(plane + (long long)z * a.pitch + L.xl, v);
   };
+  // does this lane hold ring cells of row r of s_i (their values are saved)?
+  auto ring_row = [&](int r) {
+    return MODE == 0 && a.ring_in != nullptr && r >= 0 && r < nz && lane_ring_row(a.ring, r, L);
+  };
+  // (one offset per row for all the fields: a pointer per field costs 20 registers)
   auto fetch = [&](int slot, int r) {
-    float* d = pre + slot * BWD_PRE_ROWS * 128;
-    cp_row(d + 0 * 128, MODE == 0 ? S[0] : a.v_in[0] + fb, r);
-    cp_row(d + 1 * 128, MODE == 0 ? S[1] : a.v_in[1] + fb, r);
-    cp_row(d + 2 * 128, S[2], r);
-    cp_row(d + 3 * 128, S[3], r);
-    cp_row(d + 4 * 128, A[0], r);
-    cp_row(d + 5 * 128, A[2], r);
-    cp_row(d + 6 * 128, A[3], r);
-    cp_row(d + 7 * 128, A[4], r);
-    cp_row(d + 8 * 128, S[4], r + 1);
-    cp_row(d + 9 * 128, A[1], r + 1);
+    float* d = pre + slot * BWD_PRE_ROWS * 128 + 4 * L.lane;
+    const bool in0 = L.ld && r >= 0 && r < nz, in1 = L.ld && r + 1 >= 0 && r + 1 < nz;
+    const long long o0 = in0 ? fb + (long long)r * a.pitch + L.xl : 0;
+    const long long o1 = in1 ? fb + (long long)(r + 1) * a.pitch + L.xl : 0;
+    const int n0 = in0 ? 16 : 0, n1 = in1 ? 16 : 0;
+    cp_async16(d + 0 * 128, (MODE == 0 ? a.s_in[0] : a.v_in[0]) + o0, n0);
+    cp_async16(d + 1 * 128, (MODE == 0 ? a.s_in[1] : a.v_in[1]) + o0, n0);
+    cp_async16(d + 2 * 128, a.s_in[2] + o0, n0);
+    cp_async16(d + 3 * 128, a.s_in[3] + o0, n0);
+    cp_async16(d + 4 * 128, a.a_in[0] + o0, n0);
+    cp_async16(d + 5 * 128, a.a_in[2] + o0, n0);
+    cp_async16(d + 6 * 128, a.a_in[3] + o0, n0);
+    cp_async16(d + 7 * 128, a.a_in[4] + o0, n0);
+    cp_async16(d + 8 * 128, a.s_in[4] + o1, n1);
+    cp_async16(d + 9 * 128, a.a_in[1] + o1, n1);
     if (MODE == 1) {
-      const bool wrr = r >= z0 && r < z1;  // gradient rows are only read where this warp writes them
-      cp_row(d + 10 * 128, a.grad[0] + fb, wrr ? r : -1);
-      cp_row(d + 11 * 128, a.grad[1] + fb, wrr ? r : -1);
-      cp_row(d + 12 * 128, a.grad[2] + fb, wrr ? r : -1);
+      const int ng = r >= z0 && r < z1 ? n0 : 0;  // gradient rows are only read where this warp writes them
+      cp_async16(d + 10 * 128, a.grad[0] + o0, ng);
+      cp_async16(d + 11 * 128, a.grad[1] + o0, ng);
+      cp_async16(d + 12 * 128, a.grad[2] + o0, ng);
+    } else if (ring_row(r)) {
+      const float* rb = a.ring_in + (long long)b * a.ring.size;
+#pragma unroll 1
+      for (int k = 0; k < 4; ++k) {
+        const int x = L.xl + k;
+        const int i = x >= 0 && x < a.nx ? a.ring.index(r, x) : -1;
+#pragma unroll
+        for (int f = 0; f < 5; ++f)
+          cp_async4(d + (10 + f) * 128 + k, i >= 0 ? rb + (long long)f * a.nshots * a.ring.size + i : rb, i >= 0 ? 4 : 0);
+      }
     }
     cp_async_commit();
   };
-  auto ringv = [&](int f, int z, unsigned m) {  // ring values of s_i for the components in m
-    float4 v = f4(0.f);
-    if (a.ring_in != nullptr && m != 0u) {
-      const float* rb = a.ring_in + ((long long)f * a.nshots + b) * a.ring.size;
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (m & (1u << k)) set_comp(v, k, rb[a.ring.index(z, L.xl + k)]);
-    }
-    return v;
-  };
-  auto ring_mask = [&](int z) -> unsigned {
-    if (MODE != 0 || !lane_ring_row(a.ring, z, L)) return 0u;
-    unsigned m = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int x = L.xl + k;
-      if (x >= 0 && x < a.nx && a.ring.index(z, x) >= 0) m |= 1u << k;
-    }
-    return m;
-  };
-
   // carries from row r - 1
   float4 vxi_p = f4(0.f), vzi_p = f4(0.f), hzz_p = f4(0.f), tzz_p = f4(0.f), gx_p = f4(0.f);
   float4 avxpart_p = f4(0.f), txxpart_p = f4(0.f), tzzpart_p = f4(0.f), pa_p = f4(0.f), la_p = f4(0.f);
@@ -512,27 +533,28 @@ __global__ void __launch_bounds__(128) elastic_bwd_kernel(const ElBwdArgs a) {
     const float4 q = io.ld(a.c.q, r, L), pa = io.ld(a.c.pa, r, L), la = io.ld(a.c.la, r, L);
     const float4 ma = io.ld(a.c.ma, r, L), bv = io.ld(a.c.bv, r, L), bv_n = io.ld(a.c.bv, r + 1, L);
     asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    if (MODE == 0 && (src.any != 0u || has_rec)) fix_row(pre + slot * BWD_PRE_ROWS * 128, r);
     const float* pr_ = pre + slot * BWD_PRE_ROWS * 128 + 4 * L.lane;
     // row r
-    const float4 txx = fix_s(lds4(pr_ + 2 * 128), 2, r), tzz = fix_s(lds4(pr_ + 3 * 128), 3, r);
-    const float4 avx = fix_a(lds4(pr_ + 4 * 128), 0, r);
-    const float4 atxx = fix_a(lds4(pr_ + 5 * 128), 2, r), atzz = fix_a(lds4(pr_ + 6 * 128), 3, r);
-    const float4 atxz = fix_a(lds4(pr_ + 7 * 128), 4, r);
+    const float4 txx = lds4(pr_ + 2 * 128), tzz = lds4(pr_ + 3 * 128);
+    const float4 avx = lds4(pr_ + 4 * 128);
+    const float4 atxx = lds4(pr_ + 5 * 128), atzz = lds4(pr_ + 6 * 128);
+    const float4 atxz = lds4(pr_ + 7 * 128);
     // row r + 1 parts
-    const float4 txz_n = fix_s(lds4(pr_ + 8 * 128), 4, r + 1);
-    const float4 avz_n = fix_a(lds4(pr_ + 9 * 128), 1, r + 1);
+    const float4 txz_n = lds4(pr_ + 8 * 128);
+    const float4 avz_n = lds4(pr_ + 9 * 128);
     const float4 gz_n = bv_n * avz_n;
     const float4 gx = bv * avx;
     // velocity part: Dv(s'') and v_i
     const float4 dvx = dxp(txx, L) + (r <= nz - 2 ? txz_n - txz_r : f4(0.f));
     const float4 dvz = dxm(txz_r, L) + (r >= 1 ? tzz - tzz_p : f4(0.f));
     float4 vxi, vzi;
-    unsigned rmask = 0u;
+    const bool rg = ring_row(r);
+    auto ringv = [&](int f) { return rg ? lds4(pr_ + (10 + f) * 128) : f4(0.f); };
     if (MODE == 0) {
-      rmask = inrow ? ring_mask(r) : 0u;
-      const float4 vxs = fix_s(lds4(pr_ + 0 * 128), 0, r), vzs = fix_s(lds4(pr_ + 1 * 128), 1, r);
-      vxi = pick(box, vxs - bv * dvx, ringv(0, r, rmask));
-      vzi = pick(box, vzs - bv * dvz, ringv(1, r, rmask));
+      const float4 vxs = lds4(pr_ + 0 * 128), vzs = lds4(pr_ + 1 * 128);
+      vxi = pick(box, vxs - bv * dvx, ringv(0));
+      vzi = pick(box, vzs - bv * dvz, ringv(1));
     } else {
       vxi = lds4(pr_ + 0 * 128);
       vzi = lds4(pr_ + 1 * 128);
@@ -576,9 +598,9 @@ __global__ void __launch_bounds__(128) elastic_bwd_kernel(const ElBwdArgs a) {
       glam = fma4(Sx, E, glam);
       gmu = gmu + sel(box, fma4(2.f * atxx_m, E, atxz_m * G));
       if (MODE == 0) {
-        const float4 txz_i = pick(box, txz_r - ma * G, ringv(4, r, rmask));
-        txxpart_p = pick(box, txx - pa * E, ringv(2, r, rmask));
-        tzzpart_p = pick(box, tzz - la * E, ringv(3, r, rmask));
+        const float4 txz_i = pick(box, txz_r - ma * G, ringv(4));
+        txxpart_p = pick(box, txx - pa * E, ringv(2));
+        tzzpart_p = pick(box, tzz - la * E, ringv(3));
         io.st(a.s_out[0] + fb, r, L, vxi);
         io.st(a.s_out[1] + fb, r, L, vzi);
         io.st(a.s_out[4] + fb, r, L, txz_i);
