@@ -25,7 +25,8 @@
 // staged in shared memory), in two instantiations: tiles out of reach of
 // every strip (wi = 1 over the whole stencil, no one-way line) and tiles
 // near a strip (static shares from planes filled once per reverse loop,
-// one-way transposes gathered from the staged La1 / La2).  The same
+// one-way transposes gathered from the staged La1 / La2); on small grids the
+// second takes every tile.  The same
 // equations carry the VTI (k Lx + kz Lz, vti_habc2.py), variable-density
 // (C D(U), acoustic_rho_habc.py) and Born (the scattered field's adjoint
 // against the background's reconstruction, acoustic_lsrtm_habc.py)
@@ -78,7 +79,8 @@ struct HabcBwdArgs {
   int nz, nx, pitch, nshots, hw, multiple, R;
   // tile grid (ntx strips of HT_X columns, nzb bands of HT_Z rows) and the
   // block of far tiles, strips [fx0, fx1) x bands [fz0, fz1): the far
-  // launch covers that block, the near launch the frame around it
+  // launch covers that block, the near launch the frame around it (every
+  // tile, where the block is empty)
   int ntx, nzb, fx0, fx1, fz0, fz1;
   int nfar, nnear;  // tiles of each kind per shot
   long long sstride;
@@ -467,9 +469,7 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a, int tile) {
   // lie within reach of a one-way line (depth <= hw)?
   const bool near = hw > 0 && ((!mult && z0 - HN <= hw) || z0 + HT_Z + HN >= a.nz - 1 - hw ||
                                 x0 - HT_H <= hw || x0 + HT_X + HT_H >= a.nx - 1 - hw);
-  // two launches share the grid: the NEAR instantiation takes the tiles
-  // within reach of a strip, the other the rest (with none of the strip code)
-  if (near != NEAR) return;
+  if (near && !NEAR) return;  // the far launch has none of the strip code
   // interior shares of the four cells (z, x .. x+3), x a multiple of 4
   auto wi4_at = [&](int z, int x) -> float4 {
     if (!near) return make_float4(1.f, 1.f, 1.f, 1.f);
@@ -895,15 +895,12 @@ constexpr int habc_bwd_min_blocks() {
   if (EQ == 2) return 3;
   return R <= 2 ? 3 : 2;
 }
-// The far launch waits for the step before it; the near launch (other cells,
-// nothing of the far launch is read) starts as soon as the far CTAs have all
-// passed that wait, fills the SMs that the far launch's last wave leaves idle,
-// and waits for the far launch only before it ends, so that its completion,
-// which the next step's far launch waits for, is that of the whole step.
-// Without far tiles the near launch waits for the step before it itself.
+// Both launches of a step wait for the one before them: what a wait makes
+// visible, it makes visible to its own grid only, so the near launch cannot rely
+// on the far launch's wait for the fields of the step before.
 template <int R, int EQ, bool NEAR>
 __device__ __forceinline__ void habc_bwd_step(const HabcBwdArgs& a) {
-  if (!NEAR || a.fx1 <= a.fx0) pdl_wait();
+  pdl_wait();
   pdl_trigger();
   // Far tiles: the resident CTAs walk them (a CTA per tile paid its launch and the
   // wait above 21504 times a step on 64 shots of 500 x 1100: 141 us, walked 120).
@@ -917,7 +914,6 @@ __device__ __forceinline__ void habc_bwd_step(const HabcBwdArgs& a) {
       habc_bwd_tile<R, EQ, NEAR>(a, t);
     }
   }
-  if (NEAR) pdl_wait();
 }
 template <int R, int EQ, bool NEAR>
 __global__ void __launch_bounds__(256) habc_bwd_tile_kernel(const HabcBwdArgs a) {
@@ -955,17 +951,22 @@ cudaError_t launch_habc_shares(const sgb_grid& g, const sgb_acoustic_model& m, f
   return cudaGetLastError();
 }
 
+static int sm_count() {
+  int dev = 0, sms = 152;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
 // A CTA per tile, or (walk) as many as are resident.
 template <auto KERN>
 static cudaError_t launch_tiles(int tiles, bool walk, cudaStream_t s, const HabcBwdArgs& a) {
   if (!walk) return launch_pdl(KERN, dim3((unsigned)tiles), dim3(32, HT_Z), 0, s, a);
   static int cap = 0;
   if (cap == 0) {
-    int nb = 0, dev = 0, sms = 152;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int nb = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, KERN, 32 * HT_Z, 0) != cudaSuccess || nb < 1) nb = 1;
-    cap = nb * sms;
+    cap = nb * sm_count();
   }
   return launch_pdl(KERN, dim3((unsigned)(tiles < cap ? tiles : cap)), dim3(32, HT_Z), 0, s, a);
 }
@@ -1042,7 +1043,14 @@ cudaError_t launch_habc_bwd(const sgb_grid& g, const sgb_acoustic_model& m, cons
   while (a.fx0 < a.ntx && near_strip(a.fx0)) ++a.fx0;
   a.fx1 = a.fx0;
   while (a.fx1 < a.ntx && !near_strip(a.fx1)) ++a.fx1;
-  if (a.fz1 == a.fz0 || a.fx1 == a.fx0) {  // no far tiles
+  // Few tiles: all of them in the near launch (a far tile's shares are 1, its one-way
+  // sums 0).  Up to six waves of its four CTAs per SM one launch and one wait are
+  // less than the strip code costs the far tiles: 7.3 us a step against 10.0 on one
+  // shot of 201 x 401, 11.9 against 14.1 on 8 of 228 x 356, 36.5 against 37.9 on 16
+  // of 356 x 612 (3600 tiles), but 43.4 against 41.7 on 8 of 500 x 1100 (4536) and
+  // 311 against 273 on 64.
+  const bool few = a.hw > 0 && (long long)a.ntx * a.nzb * a.nshots <= 6LL * 4 * sm_count();
+  if (few || a.fz1 == a.fz0 || a.fx1 == a.fx0) {  // no tiles for the far launch
     a.fz0 = a.fz1 = a.nzb;
     a.fx0 = a.fx1 = 0;
   }
