@@ -73,6 +73,7 @@ struct AcVjpArgs {
 struct AcStreamArgs {
   int nz, nx, pitch, nshots, ntx, zc, nzc;
   int variant;  // host: the compiled variant of the launch (fwd_variant)
+  int first;    // host: the loop's first step (not launched as a dependent)
   const float* __restrict__ um;   // U_{n-1}
   const float* __restrict__ g;    // coefficient planes
   const float* __restrict__ k;
@@ -130,6 +131,7 @@ struct AcFwdBatch {
 // as nu = k * Lambda.
 struct AcBwdStreamArgs {
   int nz, nx, pitch, nshots, ntx, zc, nzc;
+  int first;  // host: the loop's first step (not launched as a dependent)
   const float* __restrict__ unext;  // U_j
   const float* __restrict__ n2;     // nu_{j+2}
   const float* __restrict__ g;

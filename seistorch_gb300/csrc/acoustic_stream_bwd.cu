@@ -251,8 +251,8 @@ static cudaError_t bwd_tile_t(const CUtensorMap* maps, const AcBwdStreamArgs& a,
     blocks = resident_blocks(kern, 32 * NWP, smem);
   }
   const int tiles = a.nshots * a.ntx * a.nzc;
-  return launch_pdl(kern, dim3((unsigned)(tiles < blocks ? tiles : blocks)), dim3(32 * NWP), smem, s, maps[0], maps[1],
-                    maps[2], maps[3], maps[4], a);
+  return launch_step(!a.first, kern, dim3((unsigned)(tiles < blocks ? tiles : blocks)), dim3(32 * NWP), smem, s, maps[0],
+                     maps[1], maps[2], maps[3], maps[4], a);
 }
 
 template <int R>

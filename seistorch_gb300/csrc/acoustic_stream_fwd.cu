@@ -478,8 +478,8 @@ static cudaError_t fwd_tile_t(const AcFwdBatch<MAXG>& b, cudaStream_t s, bool pr
     const AcStreamArgs& a = b.g[0];
     const int tiles = a.nshots * a.ntx * a.nzc;
     if (tiles <= 0) return cudaSuccess;
-    return launch_pdl(kern, dim3((unsigned)(tiles < blocks ? tiles : blocks)), dim3(32 * NWP), smem, s, b.tm_u[0],
-                      b.tm_um[0], b.g[0]);
+    return launch_step(!a.first, kern, dim3((unsigned)(tiles < blocks ? tiles : blocks)), dim3(32 * NWP), smem, s,
+                       b.tm_u[0], b.tm_um[0], a);
   } else {
     auto kern = acoustic_fwd_batch_kernel<R, TZ, NWP, S, PT, MAXG>;
     if (blocks == 0) {
@@ -490,7 +490,8 @@ static cudaError_t fwd_tile_t(const AcFwdBatch<MAXG>& b, cudaStream_t s, bool pr
     if (prepare_only) return cudaSuccess;
     const int tiles = b.tile0[b.ngroups];
     if (tiles <= 0) return cudaSuccess;
-    return launch_pdl(kern, dim3((unsigned)(tiles < blocks ? tiles : blocks)), dim3(32 * NWP), smem, s, b);
+    return launch_step(!b.g[0].first, kern, dim3((unsigned)(tiles < blocks ? tiles : blocks)), dim3(32 * NWP), smem, s,
+                       b);
   }
 }
 

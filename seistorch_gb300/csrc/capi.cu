@@ -512,6 +512,7 @@ int acoustic_forward_impl(const sgb_grid* grid, const sgb_acoustic_model* model,
     sa.um = buf[prev];
     sa.u = buf[cur];
     sa.t = t;
+    sa.first = t == 0;
     sa.records = acq->records ? acq->records + (long long)t * acq->nrec * acq->nch : nullptr;
     // the step saves the ring of its input U_t into slot t-1 (the adjoint
     // reads the rings of U_1 .. U_{nt-2})
@@ -622,6 +623,7 @@ int sgb_born_forward(const sgb_grid* grid, const sgb_acoustic_model* model, cons
     sp.um = pbuf[prev];
     sp.un = pbuf[nxt];
     sp.t = t;
+    sp.first = t == 0;
     // the background step saves the ring of its input U_t into slot t-1
     sp.ring_src = pbuf[cur];
     sp.ring_dst = (bs != nullptr && t >= 1) ? bs->ring_store + (long long)(t - 1) * grid->nshots * ring.size : nullptr;
@@ -905,6 +907,7 @@ int acoustic_backward_impl(const sgb_grid* grid, const sgb_acoustic_model* model
     sb.unext = ubuf[uj];
     sb.n2 = lbuf[l2];
     sb.do_recon = j >= 3;
+    sb.first = j == nt;
     sb.t_src = j - 1;
     sb.resid = acq->records ? acq->records + (long long)(j - 1) * acq->nrec * acq->nch : nullptr;
     const CUtensorMap maps[5] = {uf[ujm1], nf[l1], up[uj], np[l2], cm};

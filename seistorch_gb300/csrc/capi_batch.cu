@@ -136,6 +136,7 @@ int run_batch(const sgb_batch_group* groups, int ng, int32_t* cur_out, int32_t* 
       a.um = G.buf[prev];
       a.un = G.buf[nxt];
       a.t = t;
+      a.first = t == 0;
       a.records = G.acq.records ? G.acq.records + (long long)t * G.acq.nrec * G.acq.nch : nullptr;
       b.g[k] = a;
       b.tile0[k + 1] = b.tile0[k] + a.nshots * a.ntx * a.nzc;

@@ -164,6 +164,9 @@ int set_cuda_error(cudaError_t e);
 // it wrote (the wait ends when the previous grid has completed and its writes
 // are visible) and pdl_trigger() after it, so that at most one later grid
 // waits at a time and a grid's completion implies that of every earlier one.
+// The acoustic tile kernels load what no step writes (coefficients, tables,
+// residuals) before the wait; a caller's kernel may have written that just
+// before the loop, so a loop's first step is launched without the attribute.
 // What it bounds: the gap and ramp between two steps, 2.4 us of a step's 8.3 us
 // on 8 shots of 228 x 356 (1000 forward steps 8.29 -> 6.52 ms), of 10.0 us on
 // one shot of 201 x 401 (400 steps and their adjoint 8.00 -> 5.34 ms), and of
@@ -193,8 +196,11 @@ __device__ __forceinline__ float4 ldf4(const float* p) {  // p 16-byte aligned
   return v;
 }
 
+// dependent: as a programmatic dependent of what precedes on the stream, else
+// after all of that has completed.
 template <class... P, class... A>
-inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A&... args) {
+inline cudaError_t launch_step(bool dependent, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                               const A&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -204,8 +210,12 @@ inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t 
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = dependent ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+template <class... P, class... A>
+inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A&... args) {
+  return launch_step(true, kern, grid, block, smem, s, args...);
 }
 
 // p[0..3] += v as one 16-byte reduction in L2 (p 16-byte aligned): the
