@@ -604,8 +604,9 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a, int tile) {
   // one-way transposes of the left (SX = 1) or right (SX = -1) side at the
   // lane's four cells: strip cells p = q, q - d, q - 2d (staged La1 / La2), whose
   // columns are the lane's group and the one before it along d, so that shares
-  // and velocities are two 16-byte rows (a cell beyond the strip has share 0),
-  // and the wrap of the line's depth hw-1 cell into its edge cell (global).
+  // and velocities are two 16-byte rows, and the wrap of the line's depth hw-1
+  // cell into its edge cell (global).  A cell of share 0 takes no part: beyond the
+  // strip its fields may be infinite, beyond column nx its velocity is no data.
   // Cell by cell, the strips' warps issued about 1200 instructions per row.
   auto share_cols = [&](int sd, int px) -> float4 {
     float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -636,15 +637,15 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a, int tile) {
       float t = 0.f;
       {
         const float ws = at(w0, w1, i), c = at(c0, c1, i), lam = c * a.lamf, mu = c * c * a.muf;
-        t += ws * ((2.f - lam - mu) * s_l1[rr][cx + m] + (lam - 1.f) * s_l2[rr][cx + m]);
+        if (ws != 0.f) t += ws * ((2.f - lam - mu) * s_l1[rr][cx + m] + (lam - 1.f) * s_l2[rr][cx + m]);
       }
       {
         const float ws = at(w0, w1, i - 1), c = at(c0, c1, i - 1), lam = c * a.lamf, mu = c * c * a.muf;
-        t += ws * ((lam + 2.f * mu) * s_l1[rr][cx + m - SX] - lam * s_l2[rr][cx + m - SX]);
+        if (ws != 0.f) t += ws * ((lam + 2.f * mu) * s_l1[rr][cx + m - SX] - lam * s_l2[rr][cx + m - SX]);
       }
       if (dq <= hw) {  // the depth hw-1 cell's second neighbour is the edge cell instead
         const float ws = at(w0, w1, i - 2), c = at(c0, c1, i - 2);
-        t -= ws * c * c * a.muf * s_l1[rr][cx + m - 2 * SX];
+        if (ws != 0.f) t -= ws * c * c * a.muf * s_l1[rr][cx + m - 2 * SX];
       }
       if (dq == 0) {
         const int px = xm + (hw - 1) * SX;
