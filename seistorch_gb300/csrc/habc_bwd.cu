@@ -737,7 +737,7 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a, int tile) {
     float lap, lu, luz = 0.f;
     if (RHO) {
       const float bl = m == 0 ? bxpL : comp(bxp, m - 1);
-      const float br = m == 3 ? bxnR : comp(bxn, m + 1);
+      const float br = xm + 1 >= a.nx ? 0.f : m == 3 ? bxnR : comp(bxn, m + 1);  // (padding is no data)
       lap = -(comp(bxp, m) + comp(bxn, m) + comp(bzp, m) + comp(bzn, m)) * s_kl[rr][cx + m] +
             bl * s_kl[rr][cx + m - 1] + br * s_kl[rr][cx + m + 1] + comp(bzpU, m) * s_kl[rr - 1][cx + m] +
             comp(bznD, m) * s_kl[rr + 1][cx + m];

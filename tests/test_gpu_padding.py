@@ -75,7 +75,7 @@ def _run(eq, order, nz, nx, planes, dev):
 
 @pytest.mark.parametrize("nx", [133, 134, 135])
 @pytest.mark.parametrize("eq,order,planes", [("pml", 4, True), ("habc", 2, True), ("habc", 2, False), ("habc", 8, True),
-                                             ("born", 2, True), ("vti", 2, True), ("vac", 2, True),
+                                             ("born", 2, True), ("vti", 2, True), ("rho", 2, True), ("vac", 2, True),
                                              ("elastic", 2, True)])
 def test_padding_is_never_data(dev, monkeypatch, eq, order, planes, nx):
     from seistorch_gb300 import elastic_engine, engine
