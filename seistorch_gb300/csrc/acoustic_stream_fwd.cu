@@ -519,14 +519,19 @@ static cudaError_t fwd_dispatch(int R, const AcFwdBatch<MAXG>& b, cudaStream_t s
   return cudaErrorInvalidValue;
 }
 
-// The selected variant; in place of the default (16-row tiles, best from two
-// waves of CTAs on) 8-row tiles for grids below that, where a step is the
-// latency of a tile: 4.6 against 5.6 us on 8 shots of 228 x 356 (360 tiles of 16
-// rows), 6.9 against 7.2 on 8 of 356 x 612 (920), but 19.5 against 16.0 on 32 of
-// them (3680).  nshots = 0: a batch of grids, which keeps the selected variant.
+// The variant of a launch.  A selected one is taken as it is.  Else 16-row tiles,
+// which are best from two waves of their CTAs on (four per SM), and 8-row tiles for
+// grids below that, where a step is the latency of a tile: 4.6 against 5.6 us on 8
+// shots of 228 x 356 (360 tiles of 16 rows), 6.9 against 7.2 on 8 of 356 x 612 (920),
+// but 19.5 against 16.0 on 32 of them (3680).  nshots = 0: a batch of grids, which
+// takes 16-row tiles.
 int fwd_variant(int nshots, int nz, int nx) {
+  if (g_fwd_cfg != SGB_VARIANT_AUTO) return g_fwd_cfg;
+  int dev = 0, sms = 152;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long tiles = (long long)nshots * ((nx + TX - 1) / TX) * ((nz + 15) / 16);
-  return g_fwd_cfg == 4 && nshots > 0 && tiles <= 2 * 608 ? 5 : g_fwd_cfg;
+  return nshots > 0 && tiles <= 2LL * 4 * sms ? 5 : 4;
 }
 int fwd_tile_rows(int variant) { return FWD_TILE_CFGS[variant].tz; }
 int stencil_box_width(int R) { return (R % 2 == 0) ? TX + 8 : TX + 16; }
@@ -584,7 +589,7 @@ cudaError_t launch_acoustic_fwd_batch(int R, const AcFwdBatch<MAX_BATCH_GROUPS>&
 cudaError_t prepare_acoustic_fwd_batch(int R) {
   AcFwdBatch<MAX_BATCH_GROUPS> b;
   b.ngroups = 0;
-  b.g[0].variant = g_fwd_cfg;
+  b.g[0].variant = fwd_variant(0, 0, 0);
   b.tile0[0] = 0;
   return fwd_dispatch<MAX_BATCH_GROUPS>(R, b, nullptr, true);
 }

@@ -95,7 +95,7 @@ int run_batch(const sgb_batch_group* groups, int ng, int32_t* cur_out, int32_t* 
   for (int g = 0; g < ng; ++g)
     if (int e = check_group(groups[g], order)) return e;
   const int R = order / 2;
-  const int variant = fwd_variant(0, 0, 0);  // one for the batch: the selected one
+  const int variant = fwd_variant(0, 0, 0);  // one for the batch
   const int tzr = fwd_tile_rows(variant);
   const int bw = stencil_box_width(R);
   std::vector<GroupMaps> maps(ng);

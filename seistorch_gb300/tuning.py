@@ -7,7 +7,8 @@ number of tiles against the 152 SMs, the share of halo rows, L2 reuse of
 the coefficient planes.  ``tune_grid`` times every variant on a short
 synthetic run of the given shape (CUDA events on the current stream, after
 a warm-up) and caches the winner per (nz, nx, shots, order); ``select``
-makes a winner current for the process (``sgb_set_stream_config``).  An
+makes a winner current for the process (``sgb_set_stream_config``).  Until
+then the forward's variant follows the size of each grid (``AUTO``).  An
 uneven batch of several grids runs in one persistent launch and therefore
 one variant: ``tune_batch`` times the per-grid winners on the batch itself.
 """
@@ -23,13 +24,15 @@ FWD_VARIANTS = [  # (rows per tile, warps, stages, previous field via TMA)
     (16, 4, 3, False), (16, 4, 3, True), (8, 4, 4, True), (32, 8, 2, True), (16, 4, 2, True), (8, 4, 3, True)]
 BWD_VARIANTS = [  # (rows per tile, warps, stages, point rows via TMA: 0 none, 1 U_j and nu_{j+2}, 2 also g, k)
     (8, 4, 2, 0), (8, 2, 2, 0), (16, 4, 2, 0), (8, 4, 3, 0), (8, 4, 2, 1), (8, 4, 2, 2)]
-DEFAULT = (4, 4)
+DEFAULT = (4, 4)  # best on large grids
+AUTO = 255        # SGB_VARIANT_AUTO, for the forward: what a process starts with, next to DEFAULT[1]
 
 _CACHE = {}
 
 
 def select(fwd_cfg, bwd_cfg):
-    """Make (fwd_cfg, bwd_cfg) the variants of later PML calls in this process."""
+    """Make (fwd_cfg, bwd_cfg) the variants of later PML calls in this process;
+    ``select(AUTO, DEFAULT[1])`` is the state it started in."""
     N.call("sgb_set_stream_config", int(fwd_cfg), int(bwd_cfg), 0)
 
 
