@@ -380,10 +380,13 @@ __global__ void __launch_bounds__(256) vec_scalar_wgrad_kernel(int h, int w, int
 #pragma unroll
       for (int k = 0; k < 9; ++k) acc[i][k][j] = 0.f;
   }
+  float zero = 0.f;  // NaN after an infinity or NaN of the image
   for (int q = threadIdx.x; q < TILE; q += 256) {
     const int i = q / ((VS_ROWS + 2) * TW), rr = q / TW % (VS_ROWS + 2), cc = q % TW;
     const int yy = y0 - 1 + rr, xx = blockIdx.x % ntx * VS_X - 1 + cc;
-    sm[q] = (yy >= 0 && yy < h && xx >= 0 && xx < w) ? img[i * hw + (long long)yy * w + xx] : 0.f;
+    const float u = (yy >= 0 && yy < h && xx >= 0 && xx < w) ? img[i * hw + (long long)yy * w + xx] : 0.f;
+    sm[q] = u;
+    zero = fmaf(u, 0.f, zero);
   }
   __syncthreads();
   const float* tile = sm + threadIdx.x / CG;
@@ -412,6 +415,37 @@ __global__ void __launch_bounds__(256) vec_scalar_wgrad_kernel(int h, int w, int
             const int t = SIGN > 0 ? k : 8 - k;
             acc[i][k][j] = fmaf(f[r][j], win[i][r + t / 3][t % 3], acc[i][k][j]);
           }
+      }
+    }
+  }
+  // The loop above also multiplies what takes no part: pixels beyond the images, and
+  // for the input convolution zero gradients.  That adds 0 where all is finite; else
+  // (a sum of v, or `zero`, shows it) the sums are taken again without.
+  bool redo = !(zero == 0.f);
+#pragma unroll
+  for (int j = 0; j < VS_C; ++j) redo |= !(bias[j] - bias[j] == 0.f);
+  if (__syncthreads_or(redo)) {
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+      for (int k = 0; k < 9; ++k)
+#pragma unroll
+        for (int j = 0; j < VS_C; ++j) acc[i][k][j] = 0.f;
+#pragma unroll 1
+    for (int r = 0; r < VS_ROWS && y0 + r < h; ++r) {
+      float f[VS_C];
+      vec(r, f);
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        const int t = SIGN > 0 ? k : 8 - k, yy = y0 + r - 1 + t / 3, xx = x - 1 + t % 3;
+        if (!in || yy < 0 || yy >= h || xx < 0 || xx >= w) continue;
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+          const float u = tile[(i * (VS_ROWS + 2) + r + t / 3) * TW + t % 3];
+#pragma unroll
+          for (int j = 0; j < VS_C; ++j)
+            if (SIGN < 0 || f[j] != 0.f) acc[i][k][j] = fmaf(f[j], u, acc[i][k][j]);
+        }
       }
     }
   }
