@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(128) conv_in_fwd_kernel(int n, int h, int w, i
           wt[4] = q1.x; wt[5] = q1.y; wt[6] = q1.z; wt[7] = q1.w;
         } else {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) wt[j] = t < 0 ? __ldg(b + c8 + j) : __ldg(W + (c8 + j) * 18 + t);
+          for (int j = 0; j < 8; ++j) wt[j] = t < 0 ? b[c8 + j] : W[(c8 + j) * 18 + t];  // plain loads, see ld8
         }
 #pragma unroll
         for (int k = 0; k < CIN_PX; ++k)
