@@ -28,6 +28,7 @@
 #include "sgb_common.cuh"
 #include "tma.cuh"
 #include "nn_epilogue.cuh"
+#include "row_ring.cuh"
 
 namespace sgb {
 namespace nn {
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(192) nn_conv_row_kernel(const __grid_constant_
     const uint32_t el = elect_one();
     const uint32_t idesc = mma_idesc_bf16(128, BN);
     const uint32_t wbase = smem_u32(base), rbase = smem_u32(rows);
-    int r = 0;  // rows waited for
+    int r = 0;  // rows that have arrived
     // every decision is warp-uniform: the MMAs are issued by one lane of a converged warp
     auto wait = [&](uint64_t* bar, int parity) -> bool {
       return __all_sync(0xffffffffu, !*fail && mbar_wait(bar, parity, g.status));
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(192) nn_conv_row_kernel(const __grid_constant_
     for (int t = t0, lt = 0; t < t1 && ok; ++t, ++lt) {
       const int y = t % g.H, buf = lt & 1;
       const int need = (t == t0 || y == 0) ? 3 : 1;
-      for (int i = 0; i < need && ok; ++i, ++r) ok = wait(&full[r % R], (r / R) & 1);
+      ok = take_rows(need, r, [&](int row) { return wait(&full[row % R], (row / R) & 1); });
       if (ok && lt >= 2) ok = wait(&acc_empty[buf], ((lt >> 1) - 1) & 1);
       if (!ok) break;
       tc_fence_after();
