@@ -36,12 +36,12 @@ int make_tmap_f32(CUtensorMap* map, const float* base, int rank, const uint64_t*
   return r == CUDA_SUCCESS ? 0 : -2;
 }
 
-// Tensor maps of a [nshots][nz][pitch] field with a box of boxw columns,
-// rb rows and bs shots.
-int field_map(CUtensorMap* m, const float* p, int nz, int nx, int pitch, int nshots, int boxw, int rb, int bs) {
+// Tensor maps of a [nshots][nz][pitch] field with a box of boxw columns and rb
+// rows of one shot.
+int field_map(CUtensorMap* m, const float* p, int nz, int nx, int pitch, int nshots, int boxw, int rb) {
   const uint64_t dims[3] = {(uint64_t)nx, (uint64_t)nz, (uint64_t)nshots};
   const uint64_t st[2] = {(uint64_t)pitch * 4, (uint64_t)nz * pitch * 4};
-  const uint32_t box[3] = {(uint32_t)boxw, (uint32_t)rb, (uint32_t)bs};
+  const uint32_t box[3] = {(uint32_t)boxw, (uint32_t)rb, 1};
   return make_tmap_f32(m, p, 3, dims, st, box);
 }
 int coef_map(CUtensorMap* m, const float* coef, int nz, int nx, int pitch, int rb) {
@@ -49,12 +49,6 @@ int coef_map(CUtensorMap* m, const float* coef, int nz, int nx, int pitch, int r
   const uint64_t st[2] = {(uint64_t)pitch * 4, (uint64_t)nz * pitch * 4};
   const uint32_t box[3] = {(uint32_t)TX, (uint32_t)rb, 2};
   return make_tmap_f32(m, coef, 3, dims, st, box);
-}
-int plane_map(CUtensorMap* m, const float* p, int nz, int nx, int pitch, int boxw, int rb) {
-  const uint64_t dims[2] = {(uint64_t)nx, (uint64_t)nz};
-  const uint64_t st[1] = {(uint64_t)pitch * 4};
-  const uint32_t box[2] = {(uint32_t)boxw, (uint32_t)rb};
-  return make_tmap_f32(m, p, 2, dims, st, box);
 }
 
 // Variant selection: fwd_cfg / bwd_cfg index the (rows per tile, warps per

@@ -16,7 +16,7 @@
 //     shot-point and step);
 //   * the reconstruction U_{j-2} = 2 U_{j-1} - (U_j - S w_{j-1}) + k L(U_{j-1})
 //     inside the box (g = 2 there), the saved ring around it (each CTA
-//     copies a share after its tiles), 0 in the damped band.
+//     copies a share while its first boxes load), 0 in the damped band.
 #include "stream_common.cuh"
 
 namespace sgb {

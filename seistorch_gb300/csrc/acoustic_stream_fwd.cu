@@ -225,8 +225,7 @@ __device__ __forceinline__ void fwd_tiles(const P& prov, const Pre& pre = Pre{})
     const int zw = g.z0 + wid * RPW;  // first row of this warp
     const int b = g.b;
     const long long fbase = (long long)b * a.sstride;
-    // point operands of this warp's rows, issued before the stage wait (the
-    // coefficient rows serve every shot of the tile)
+    // point operands of this warp's rows, issued before the stage wait
     float4 vm[RPW], vg[RPW], vk[RPW];
     float4 vkz[HB == 2 ? RPW : 1];  // VTI: the kz rows as well
     float4 vrc[HB == 3 ? RPW : 1][5];  // variable density: the C, bx+, bx-, bz+, bz- rows

@@ -83,10 +83,8 @@ struct VacParams {
 };
 cudaError_t launch_acoustic_bwd_stream(int R, const CUtensorMap* maps, const AcBwdStreamArgs& a,
                                        cudaStream_t s);
-int field_map(CUtensorMap* m, const float* p, int nz, int nx, int pitch, int nshots, int boxw, int rb,
-              int bs = 1);
+int field_map(CUtensorMap* m, const float* p, int nz, int nx, int pitch, int nshots, int boxw, int rb);
 int coef_map(CUtensorMap* m, const float* coef, int nz, int nx, int pitch, int rb);
-int plane_map(CUtensorMap* m, const float* p, int nz, int nx, int pitch, int boxw, int rb);
 int fwd_variant(int nshots, int nz, int nx);
 int fwd_tile_rows(int variant);
 int bwd_tile_rows();

@@ -11,8 +11,7 @@
 
 namespace sgb {
 FdWeights fd_weights(int order);
-int field_map(CUtensorMap* m, const float* p, int nz, int nx, int pitch, int nshots, int boxw, int rb,
-              int bs = 1);
+int field_map(CUtensorMap* m, const float* p, int nz, int nx, int pitch, int nshots, int boxw, int rb);
 int fwd_variant(int nshots, int nz, int nx);
 int fwd_tile_rows(int variant);
 int stencil_box_width(int R);

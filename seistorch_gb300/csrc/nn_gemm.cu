@@ -1,17 +1,10 @@
 // BF16 x BF16 -> FP32 GEMM on the 5th-generation tensor cores (tcgen05) for
 // the learned gradient preconditioner's 3x3 convolutions.
 //
-// One CTA computes a 128 x BN tile of D = sum_k A[m, k] B[n, k] (both
-// operands K-major) with the accumulator in tensor memory:
-//   warp 0         -- TMA producer (one elected lane): per K step one A box (128 rows x RB
-//                     bytes) and one B box (BN rows x RB bytes) into a stage
-//                     of an S-deep ring, 128/64-byte swizzled;
-//   warp 1         -- MMA issuer (one elected lane): RB/32 tcgen05.mma (K = 16) per stage, then
-//                     tcgen05.commit to the stage's "empty" mbarrier;
-//   all 4 warps    -- epilogue: tcgen05.ld of their 32 TMEM lanes (= rows).
-// Warp 0 allocates and frees the TMEM columns.  Every wait is bounded; on a
-// timeout the CTA records DEV_ERR_TIMEOUT, waits (bounded) for what it
-// issued and frees its TMEM before returning.
+// A tile is 128 x BN of D = sum_k A[m, k] B[n, k] (both operands K-major) with
+// the accumulator in tensor memory; the kernel below says which warp does what.
+// Every wait is bounded; on a timeout the CTA records DEV_ERR_TIMEOUT, waits
+// (bounded) for what it issued and frees its TMEM before returning.
 //
 // Two operand modes:
 //   CONV  : implicit GEMM of a 3x3 convolution (zero padding 1).  A = input
@@ -21,11 +14,12 @@
 //           the tensor map, never on the innermost one; B = weights
 //           [Cout][9][Cin].  Used for the forward pass and, with flipped
 //           transposed weights, for the data gradient.
-//   WGRAD : weight gradient of one tap (blockIdx.z % 9) and 128 output
-//           channels (blockIdx.z / 9): A = dY in CHW (rows = output channels), B = the input in CHW shifted by the tap's x
-//           offset (one of three pre-shifted copies) and read at the tap's y
-//           offset; K = pixels, split over blockIdx.x; FP32 atomics into
-//           dW[cout][cin][3][3].
+//   WGRAD : weight gradient (sgb_nn_conv3x3_wgrad, for operands already in CHW;
+//           nn_wgrad.cu takes them in NHWC) of one tap (tile z % 9) and 128
+//           output channels (tile z / 9): A = dY in CHW (rows = output channels),
+//           B = the input in CHW shifted by the tap's x offset (one of three
+//           pre-shifted copies) and read at the tap's y offset; K = pixels, split
+//           over the tiles' x; FP32 atomics into dW[cout][cin][3][3].
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <stdint.h>

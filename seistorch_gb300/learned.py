@@ -20,7 +20,7 @@ W >= 512):
 
 All 3x3 convolutions except the first and last run on the tcgen05 tensor
 cores (``sgb_nn_conv3x3``: forward and data gradient;
-``sgb_nn_conv3x3_wgrad``: weight gradient); ReLU after every hidden layer;
+``sgb_nn_conv3x3_wgrad_nhwc``: weight gradient); ReLU after every hidden layer;
 2x2 average pooling, nearest upsampling, skip concatenation by writing into
 channel slices.  Adam on fp32 master weights; the bf16 copies are repacked
 after every step.
