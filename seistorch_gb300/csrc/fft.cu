@@ -24,10 +24,11 @@
 // 7000, with a prime factor above 137) take the general kernels at the end, one
 // output of a stage at a time.
 //
-// Rounding: for every length of 100 to 1300 the error is at most that of direct
-// sums over the prime factors (of the norm 0.9 to 1.4e-7 a transform, 1.9 to 2.5e-7
-// with chirp-z).  What that takes beside the choice above is said where it stands:
-// the sine of radix 5, the chains of radix 3, the twiddles of some lengths.
+// Rounding: on white noise the operator's error is at most that of direct sums over
+// the prime factors at every length of 100 to 1300 (a transform 0.9 to 1.4e-7 of the
+// norm, with chirp-z 1.9 to 2.5e-7), on smooth fields 0.55 to 1.06 of it.  What that
+// takes beside the choice above is said where it stands: the sine of radix 5, the
+// chains of radix 3, the twiddles of some lengths.
 //
 // What bounds it: latency of the first pass' global loads and of the twiddle
 // loads (rows, 44 % of the warps resident), barriers between the passes of a
