@@ -217,8 +217,10 @@ cudaError_t launch_t(const CUtensorMap* maps, const WgradArgs& g, int splits, cu
 // of 32 / 64 output channels, and about 600 where the copies' latency, not the
 // MMAs, is what a step waits for (one tap).  128 -> 128 channels: 64 us as three
 // taps by 64, 40 us as one tap by 64; 384 -> 128: 162 us as one tap by 128 in
-// two waves, 75 us as three taps by 64 in one.  The B box of the tensor map is
-// 64 channels (32 for bn = 32).
+// two waves, 75 us as three taps by 64 in one.  Against the best variant of each of
+// the nine layers the rule is 9 % off at batch 8 of 256 x 512 (729 us in all), 9 and
+// 12 % at batch 1 and 2, 0.5 % at 4 of 384 x 1024 and 8 % at 8 of 128 x 512.  The B
+// box of the tensor map is 64 channels (32 for bn = 32).
 static void wgrad_tile(const WgradArgs& g, int splits, int* bn, int* taps) {
   const int sms = sm_count(), mt = (g.Cin + 127) / 128;
   int best = 0;
