@@ -14,6 +14,7 @@ static thread_local int g_last_cuda_error = 0;
 
 int set_cuda_error(cudaError_t e) {
   g_last_cuda_error = (int)e;
+  cudaGetLastError();  // the caller has the status: not left for its own next launch check
   return SGB_ERR_CUDA;
 }
 
