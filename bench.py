@@ -628,7 +628,7 @@ def bench_habc(args):
                        "grid": [nz, nx], "shots": shots, "nt": nt, "order": order, "ckpt_every": ck,
                        "l2": "inputs larger than L2 (141 MB per field)"},
             "shots_per_s": shots / (ms * 1e-3), "phases_ms": {"forward": fwd_ms, "adjoint": rev_ms},
-            "roofline": {"kernel": "habc_bwd_tile_kernel (far + near tiles)", "bound": "hbm", "achieved": rev_gbs,
+            "roofline": {"kernel": "habc_bwd_kernel", "bound": "hbm", "achieved": rev_gbs,
                          "peak": peak, "peak_kind": kind, "unit": "GB/s", "frac": rev_gbs / peak, "traffic": None,
                          "bytes_per_launch": rev_bytes, "launch_ms": rev_ms / (nt - 1)},
             "roofline_forward": {"kernel": "acoustic_fwd_tile_kernel<HABC>", "achieved": fwd_gbs,
@@ -929,7 +929,7 @@ def bench_born(args):
                        "grid": [nz, nx], "shots": shots, "nt": nt, "ckpt_every": ck,
                        "l2": "inputs larger than L2 (70 MB per field, 6 fields)"},
             "shots_per_s": shots / (ms * 1e-3), "phases_ms": {"forward": fwd_ms, "adjoint": rev_ms},
-            "roofline": {"kernel": "habc_bwd_tile_kernel (far + near tiles)", "bound": "hbm", "achieved": rev_gbs, "peak": peak,
+            "roofline": {"kernel": "habc_bwd_kernel", "bound": "hbm", "achieved": rev_gbs, "peak": peak,
                          "peak_kind": kind, "unit": "GB/s", "frac": rev_gbs / peak, "traffic": None,
                          "bytes_per_launch": rev_bytes, "launch_ms": rev_ms / (nt - 1)},
             "roofline_forward": {"kernel": "acoustic_fwd_tile_kernel<HABC> x2 (background, scattered)",
@@ -1030,7 +1030,7 @@ def bench_vti(args):
                        "grid": [nz, nx], "shots": shots, "nt": nt, "ckpt_every": ck,
                        "l2": "inputs larger than L2 (70 MB per field)"},
             "shots_per_s": shots / (ms_ * 1e-3), "phases_ms": {"forward": fwd_ms, "adjoint": rev_ms},
-            "roofline": {"kernel": "habc_bwd_tile_kernel (VTI, far + near tiles)", "bound": "hbm", "achieved": rev_gbs, "peak": peak,
+            "roofline": {"kernel": "habc_bwd_kernel (VTI)", "bound": "hbm", "achieved": rev_gbs, "peak": peak,
                          "peak_kind": kind, "unit": "GB/s", "frac": rev_gbs / peak, "traffic": None,
                          "bytes_per_launch": rev_bytes, "launch_ms": rev_ms / (nt - 1)},
             "roofline_forward": {"kernel": "acoustic_fwd_tile_kernel<HABC> (VTI)", "achieved": fwd_gbs,
@@ -1127,7 +1127,7 @@ def bench_rho(args):
                        "grid": [nz, nx], "shots": shots, "nt": nt, "ckpt_every": ck,
                        "l2": "inputs larger than L2 (70 MB per field)"},
             "shots_per_s": shots / (ms_ * 1e-3), "phases_ms": {"forward": fwd_ms, "adjoint": rev_ms},
-            "roofline": {"kernel": "habc_bwd_tile_kernel (variable density, far + near tiles)", "bound": "hbm", "achieved": rev_gbs,
+            "roofline": {"kernel": "habc_bwd_kernel (variable density)", "bound": "hbm", "achieved": rev_gbs,
                          "peak": peak, "peak_kind": kind, "unit": "GB/s", "frac": rev_gbs / peak, "traffic": None,
                          "bytes_per_launch": rev_bytes, "launch_ms": rev_ms / (nt - 1)},
             "roofline_forward": {"kernel": "acoustic_fwd_tile_kernel<HABC> (variable density)", "achieved": fwd_gbs,

@@ -21,12 +21,11 @@
 // dJ/dvp += La_j (2k / vp) L(U_{j-1}) there; the ring of order/2 cells
 // around the box comes from the forward's store.
 //
-// One kernel takes each reverse step (habc_bwd_tile_kernel, 8 x 128 tiles
-// staged in shared memory), in two instantiations: tiles out of reach of
-// every strip (wi = 1 over the whole stencil, no one-way line) and tiles
-// near a strip (static shares from planes filled once per reverse loop,
-// one-way transposes gathered from the staged La1 / La2); on small grids the
-// second takes every tile.  The same
+// One launch takes each reverse step (habc_bwd_kernel, 8 x 128 tiles staged in
+// shared memory), with code of their own for tiles out of reach of every strip
+// (wi = 1 over the whole stencil, no one-way line) and tiles near a strip (static
+// shares from planes filled once per reverse loop, one-way transposes gathered
+// from the staged La1 / La2).  The same
 // equations carry the VTI (k Lx + kz Lz, vti_habc2.py), variable-density
 // (C D(U), acoustic_rho_habc.py) and Born (the scattered field's adjoint
 // against the background's reconstruction, acoustic_lsrtm_habc.py)
@@ -78,11 +77,11 @@ __device__ __forceinline__ HabcW habc_weights(int z, int x, int nz, int nx, int 
 struct HabcBwdArgs {
   int nz, nx, pitch, nshots, hw, multiple, R;
   // tile grid (ntx strips of HT_X columns, nzb bands of HT_Z rows) and the
-  // block of far tiles, strips [fx0, fx1) x bands [fz0, fz1): the far
-  // launch covers that block, the near launch the frame around it (every
-  // tile, where the block is empty)
+  // block of far tiles, strips [fx0, fx1) x bands [fz0, fz1); the near tiles are
+  // the frame around it
   int ntx, nzb, fx0, fx1, fz0, fz1;
   int nfar, nnear;  // tiles of each kind per shot
+  int walkers;      // CTAs that walk the far tiles
   long long sstride;
   const float* __restrict__ la1;   // La_{j+1}
   const float* __restrict__ la2;   // La_{j+2}
@@ -418,17 +417,17 @@ __device__ __forceinline__ float4 lap_rows4(const float (*s)[W], int rr, int cx,
 }
 
 template <int R, int EQ, bool NEAR>
-__device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a, int tile) {
+__device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a, int tile, float* smem) {
   constexpr bool VTI = EQ == 1, RHO = EQ == 2;
   static_assert(!RHO || R == 1, "variable density is second order");
   // row halo: the stencil's R, and 2 for the one-way lines (q - d, q - 2d) near a strip
-  constexpr int HN = R < 2 ? 2 : R, HR = NEAR ? HN : R;
+  constexpr int HR = NEAR && R < 2 ? 2 : R;
   constexpr int ROWS = HT_Z + 2 * HR, W = HT_X + 2 * HT_H;
-  __shared__ __align__(16) float s_kl[ROWS][W];             // k wi La1 (VTI: kx wi La1; density: C wi La1)
-  __shared__ __align__(16) float s_kzl[VTI ? ROWS : 1][W];  // VTI: kz wi La1
-  __shared__ __align__(16) float s_u[ROWS][W];
-  __shared__ __align__(16) float s_l1[NEAR ? ROWS : 1][W];  // La1 and La2 (tiles near a strip only)
-  __shared__ __align__(16) float s_l2[NEAR ? ROWS : 1][W];
+  float(*const s_kl)[W] = reinterpret_cast<float(*)[W]>(smem);  // k wi La1 (VTI: kx wi La1; density: C wi La1)
+  float(*const s_u)[W] = s_kl + ROWS;
+  float(*const s_l1)[W] = s_u + ROWS;  // La1 and La2 (tiles near a strip only)
+  float(*const s_l2)[W] = s_l1 + ROWS;
+  float(*const s_kzl)[W] = NEAR ? s_l2 + ROWS : s_l1;  // VTI: kz wi La1
   // tile of this kind -> (shot, band, strip), strips fastest
   const int ntile = NEAR ? a.nnear : a.nfar;
   const int b = tile / ntile;
@@ -465,14 +464,9 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a, int tile) {
   const bool mult = a.multiple != 0;
   const long long pl = (long long)a.nz * a.pitch;
   const float* __restrict__ kp = RHO ? a.rho_c : a.k;  // the plane that weights La1
-  // does any cell of the tile or its halo have an interior share below 1, or
-  // lie within reach of a one-way line (depth <= hw)?
-  const bool near = hw > 0 && ((!mult && z0 - HN <= hw) || z0 + HT_Z + HN >= a.nz - 1 - hw ||
-                                x0 - HT_H <= hw || x0 + HT_X + HT_H >= a.nx - 1 - hw);
-  if (near && !NEAR) return;  // the far launch has none of the strip code
   // interior shares of the four cells (z, x .. x+3), x a multiple of 4
   auto wi4_at = [&](int z, int x) -> float4 {
-    if (!near) return make_float4(1.f, 1.f, 1.f, 1.f);
+    if (!NEAR) return make_float4(1.f, 1.f, 1.f, 1.f);
     const long long oo = (long long)z * a.pitch + x;
     if (a.wpl != nullptr) return __ldg(reinterpret_cast<const float4*>(a.wpl + oo));
     float4 r;
@@ -885,47 +879,39 @@ __device__ __forceinline__ void habc_bwd_tile(const HabcBwdArgs& a, int tile) {
   if (a.uout != nullptr) *reinterpret_cast<float4*>(a.uout + fb + o) = make_float4(uo[0], uo[1], uo[2], uo[3]);
 }
 
-// The plain / Born equation's far kernel is left to the compiler's register
-// choice; the others are held to a number of CTAs per SM (eight warps each):
-// near tiles four (variable density two; the plain near kernel at the 80
-// registers the compiler would take fits three: 179 us a step against 148 on 64
-// shots of 500 x 1100), far tiles three (VTI of order 6 and 8 two).
-template <int R, int EQ, bool NEAR>
-constexpr int habc_bwd_min_blocks() {
-  if (NEAR) return EQ == 2 ? 2 : 4;
-  if (EQ == 2) return 3;
-  return R <= 2 ? 3 : 2;
-}
-// Both launches of a step wait for the one before them: what a wait makes
-// visible, it makes visible to its own grid only, so the near launch cannot rely
-// on the far launch's wait for the fields of the step before.
-template <int R, int EQ, bool NEAR>
-__device__ __forceinline__ void habc_bwd_step(const HabcBwdArgs& a) {
-  pdl_wait();
-  pdl_trigger();
-  // Far tiles: the resident CTAs walk them (a CTA per tile paid its launch and the
-  // wait above 21504 times a step on 64 shots of 500 x 1100: 141 us, walked 120).
-  // Near tiles: a CTA each (148 us; walked, the loop's registers cost more, 155).
-  if constexpr (NEAR) {
-    habc_bwd_tile<R, EQ, NEAR>(a, blockIdx.x);
-  } else {
-    const int n = a.nfar * a.nshots;
-    for (int t = blockIdx.x; t < n; t += gridDim.x) {
-      if (t != (int)blockIdx.x) __syncthreads();  // the shared tile of the one before is read
-      habc_bwd_tile<R, EQ, NEAR>(a, t);
-    }
-  }
-}
-template <int R, int EQ, bool NEAR>
-__global__ void __launch_bounds__(256) habc_bwd_tile_kernel(const HabcBwdArgs a) {
-  habc_bwd_step<R, EQ, NEAR>(a);
-}
-template <int R, int EQ, bool NEAR>
-__global__ void __launch_bounds__(256, habc_bwd_min_blocks<R, EQ, NEAR>()) habc_bwd_tile_kernel_held(
-    const HabcBwdArgs a) {
-  habc_bwd_step<R, EQ, NEAR>(a);
+// Floats of shared memory of a tile near a strip (a far tile takes less).
+template <int R, int EQ>
+constexpr int habc_bwd_smem() {
+  const int rows = HT_Z + 2 * (R < 2 ? 2 : R);
+  return (EQ == 1 ? 5 : 4) * rows * (HT_X + 2 * HT_H);
 }
 
+// A reverse step: a CTA for each near tile, then a.walkers CTAs that walk the far
+// ones.  The near tiles are issue-bound and the far ones wait for memory; walkers
+// become resident as near CTAs leave, so the two overlap and the step has one tail.
+// In one grid, since a grid may rely only on its own wait for the fields of the step
+// before.  64 shots of 500 x 1100: 262 us a step, 268 as two launches; 24 of
+// 433 x 1001 82.1 (90.2), 8 of 500 x 1100 34.8 (41.4), 8 of 228 x 356 9.9 (14.1); VTI,
+// 32 of 500 x 1100 153.8 (168.9), variable density 209.0 (225.3).  With the walkers
+// first 2 % less on the first, but 20.5 against 17.7 on 4 shots and 11.6 against 10.1
+// on the last.
+// Four CTAs per SM (64 registers; at the 80 that the near tiles would take three fit:
+// 32 VTI shots 180), variable density three (80 registers; 117 and two: 243).
+template <int R, int EQ>
+__global__ void __launch_bounds__(256, EQ == 2 ? 3 : 4) habc_bwd_kernel(const HabcBwdArgs a) {
+  __shared__ __align__(16) float smem[habc_bwd_smem<R, EQ>()];
+  pdl_wait();
+  pdl_trigger();
+  const int nnear = a.nnear * a.nshots, nfar = a.nfar * a.nshots, w = (int)blockIdx.x - nnear;
+  if (w < 0) {
+    habc_bwd_tile<R, EQ, true>(a, blockIdx.x, smem);
+    return;
+  }
+  for (int t = w; t < nfar; t += a.walkers) {
+    if (t != w) __syncthreads();  // the shared tile of the one before is read
+    habc_bwd_tile<R, EQ, false>(a, t, smem);
+  }
+}
 
 // The static shares of every cell: wi and the four sides' b * share.
 __global__ void habc_shares_kernel(int nz, int nx, int pitch, int hw, int mult, const float* __restrict__ hb,
@@ -950,26 +936,6 @@ cudaError_t launch_habc_shares(const sgb_grid& g, const sgb_acoustic_model& m, f
   if (blocks > 152 * 8) blocks = 152 * 8;
   habc_shares_kernel<<<(unsigned)blocks, 256, 0, s>>>(g.nz, g.nx, g.pitch, m.habc_width, m.multiple, m.damp, planes);
   return cudaGetLastError();
-}
-
-static int sm_count() {
-  int dev = 0, sms = 152;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
-// A CTA per tile, or (walk) as many as are resident.
-template <auto KERN>
-static cudaError_t launch_tiles(int tiles, bool walk, cudaStream_t s, const HabcBwdArgs& a) {
-  if (!walk) return launch_pdl(KERN, dim3((unsigned)tiles), dim3(32, HT_Z), 0, s, a);
-  static int cap = 0;
-  if (cap == 0) {
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, KERN, 32 * HT_Z, 0) != cudaSuccess || nb < 1) nb = 1;
-    cap = nb * sm_count();
-  }
-  return launch_pdl(KERN, dim3((unsigned)(tiles < cap ? tiles : cap)), dim3(32, HT_Z), 0, s, a);
 }
 
 cudaError_t launch_habc_bwd(const sgb_grid& g, const sgb_acoustic_model& m, const sgb_acquisition& q,
@@ -1021,10 +987,10 @@ cudaError_t launch_habc_bwd(const sgb_grid& g, const sgb_acoustic_model& m, cons
   const int R = a.R;
   if (R > HT_H) return cudaErrorInvalidValue;
   const int eq = rho_c != nullptr ? 2 : (kz != nullptr ? 1 : 0);
-  if (eq == 2 && R != 1) return cudaErrorInvalidValue;  // variable density: 2nd order only
-  // the far tiles (out of reach of every strip: the kernel's own test, per
-  // band and per strip) form one block of bands x strips; the rest is the
-  // frame around it
+  if (eq != 0 && R != 1) return cudaErrorInvalidValue;  // VTI, variable density: 2nd order only
+  // the far tiles (no cell of the tile or its halo has an interior share below 1 or
+  // lies within reach of a one-way line, depth <= hw) form one block of bands x
+  // strips; the rest is the frame around it
   const int HR = R < 2 ? 2 : R;
   a.ntx = (g.nx + HT_X - 1) / HT_X;
   a.nzb = (g.nz + HT_Z - 1) / HT_Z;
@@ -1044,45 +1010,30 @@ cudaError_t launch_habc_bwd(const sgb_grid& g, const sgb_acoustic_model& m, cons
   while (a.fx0 < a.ntx && near_strip(a.fx0)) ++a.fx0;
   a.fx1 = a.fx0;
   while (a.fx1 < a.ntx && !near_strip(a.fx1)) ++a.fx1;
-  // Few tiles: all of them in the near launch (a far tile's shares are 1, its one-way
-  // sums 0).  Up to six waves of its four CTAs per SM one launch and one wait are
-  // less than the strip code costs the far tiles: 7.3 us a step against 10.0 on one
-  // shot of 201 x 401, 11.9 against 14.1 on 8 of 228 x 356, 36.5 against 37.9 on 16
-  // of 356 x 612 (3600 tiles), but 43.4 against 41.7 on 8 of 500 x 1100 (4536) and
-  // 311 against 273 on 64.
-  const bool few = a.hw > 0 && (long long)a.ntx * a.nzb * a.nshots <= 6LL * 4 * sm_count();
-  if (few || a.fz1 == a.fz0 || a.fx1 == a.fx0) {  // no tiles for the far launch
+  if (a.fz1 == a.fz0 || a.fx1 == a.fx0) {  // no far tiles
     a.fz0 = a.fz1 = a.nzb;
     a.fx0 = a.fx1 = 0;
   }
   a.nfar = (a.fx1 - a.fx0) * (a.fz1 - a.fz0);
   a.nnear = a.ntx * a.nzb - a.nfar;
-  const int nfar = a.nfar, nnear = a.nnear;
-  // one launch for the tiles out of reach of the strips, one for the rest
-  cudaError_t err = cudaSuccess;
-  switch (R * 3 + eq) {
-#define SGB_TILE2(RR, EQ)                                                                            \
-  if (nfar > 0) {                                                                                    \
-    if constexpr (EQ == 0)                                                                           \
-      err = launch_tiles<habc_bwd_tile_kernel<RR, EQ, false>>(nfar * g.nshots, true, s, a);          \
-    else                                                                                             \
-      err = launch_tiles<habc_bwd_tile_kernel_held<RR, EQ, false>>(nfar * g.nshots, true, s, a);     \
-  }                                                                                                  \
-  if (nnear > 0 && err == cudaSuccess)                                                               \
-    err = launch_tiles<habc_bwd_tile_kernel_held<RR, EQ, true>>(nnear * g.nshots, false, s, a);
-    case 3: SGB_TILE2(1, 0) break;
-    case 4: SGB_TILE2(1, 1) break;
-    case 5: SGB_TILE2(1, 2) break;
-    case 6: SGB_TILE2(2, 0) break;
-    case 7: SGB_TILE2(2, 1) break;
-    case 9: SGB_TILE2(3, 0) break;
-    case 10: SGB_TILE2(3, 1) break;
-    case 12: SGB_TILE2(4, 0) break;
-    case 13: SGB_TILE2(4, 1) break;
-#undef SGB_TILE2
-    default: return cudaErrorInvalidValue;
+  // four waves of walkers at most: fewer leave a longer tail on mid-sized grids (608 of
+  // them: 8 shots of 500 x 1100 36.7 us against 35.5), more are no faster
+  int dev = 0, sms = 152;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long long far = (long long)a.nfar * a.nshots, near = (long long)a.nnear * a.nshots;
+  a.walkers = (int)(far < 16LL * sms ? far : 16LL * sms);
+  if (far + near >= (1LL << 31) - 16LL * sms) return cudaErrorInvalidValue;  // 32-bit tile numbers
+  const dim3 grid((unsigned)(near + a.walkers)), block(32, HT_Z);
+  if (eq == 2) return launch_pdl(habc_bwd_kernel<1, 2>, grid, block, 0, s, a);
+  if (eq == 1) return launch_pdl(habc_bwd_kernel<1, 1>, grid, block, 0, s, a);
+  switch (R) {
+    case 1: return launch_pdl(habc_bwd_kernel<1, 0>, grid, block, 0, s, a);
+    case 2: return launch_pdl(habc_bwd_kernel<2, 0>, grid, block, 0, s, a);
+    case 3: return launch_pdl(habc_bwd_kernel<3, 0>, grid, block, 0, s, a);
+    case 4: return launch_pdl(habc_bwd_kernel<4, 0>, grid, block, 0, s, a);
   }
-  return err;
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_habc_step_vjp(const sgb_grid& g, const sgb_acoustic_model& m, const sgb_habc_vjp_io& io,

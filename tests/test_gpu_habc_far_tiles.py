@@ -1,7 +1,6 @@
-"""HABC reverse loops on both sides of the rule that sends every tile to one
-launch: enough shots for two launches a step with one to four far tiles each (most
-SMs then run tiles of the frame only), and groups of those shots small enough for
-one launch.
+"""HABC reverse loops whose launch holds many times the tiles that are resident:
+shots with one to four far tiles each (most CTAs then take tiles of the frame), with
+more far tiles than CTAs that walk them, and groups of few shots.
 
 Whole-loop gradients against the step-by-step loop under autograd (its single-step
 VJP is another kernel) and against the sum of the groups' gradients.  All are fp32
@@ -39,21 +38,12 @@ def _survey(nz, nx, multiple, shots, dev):
     return vp, b, ricker_wave(30.0, DT, NT, delay=30), src, (top + 3, rx), (slice(top, nz - W), slice(W, nx - W))
 
 
-def _tiles(nz, nx, shots):
-    return shots * ((nz + 7) // 8) * ((nx + 127) // 128)
-
-
-def _limit(dev):
-    return 24 * torch.cuda.get_device_properties(dev).multi_processor_count
-
-
 @pytest.mark.parametrize("nz,nx,multiple,shots,ckpt", [(118, 312, False, 82, 0), (118, 441, False, 62, 16),
                                                        (70, 315, True, 136, 16)])
 def test_gradient_with_few_far_tiles_a_shot(dev, nz, nx, multiple, shots, ckpt):
     from seistorch_gb300 import engine
     from seistorch_gb300.equations2d import acoustic_habc
     from seistorch_gb300.habc import bound_mask
-    assert _tiles(nz, nx, shots) > _limit(dev)
     vp0, b, wav, src, (rz, rx), box = _survey(nz, nx, multiple, shots, dev)
     prop = engine.AcousticPropagator(nz, nx, DT, H, 2, "habc", W, multiple, dev)
     acq = engine.Acquisition(nz, nx, src, [([rz] * len(rx), rx)] * shots, wav, dev)
@@ -79,10 +69,12 @@ def test_gradient_with_few_far_tiles_a_shot(dev, nz, nx, multiple, shots, ckpt):
 
 @pytest.mark.parametrize("eq,order", [("habc", 2), ("habc", 4), ("habc", 6), ("habc", 8), ("born", 2), ("vti", 2),
                                       ("rho", 2)])
-def test_one_launch_and_two_agree(dev, eq, order):
+def test_groups_of_shots_agree(dev, eq, order):
     from seistorch_gb300 import engine
-    nz, nx, shots = 131, 427, 57  # two launches for all the shots, one for a third of them
-    assert _tiles(nz, nx, shots) > _limit(dev) >= _tiles(nz, nx, shots // 3)
+    # 34 far tiles a shot: a CTA walks several in the whole batch, one in a group of an eighth
+    nz, nx, shots, groups = 251, 441, 80, 8
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    assert 34 * shots > 16 * sms > 34 * shots // groups
     vp0, b, wav, src, (rz, rx), box = _survey(nz, nx, False, shots, dev)
     par = [vp0]
     if eq == "born":
@@ -108,6 +100,6 @@ def test_one_launch_and_two_agree(dev, eq, order):
         return [t.grad[box].double().cpu().numpy() for t in p]
 
     whole = gradient(src)
-    parts = [gradient(src[k:k + shots // 3]) for k in range(0, shots, shots // 3)]
+    parts = [gradient(src[k:k + shots // groups]) for k in range(0, shots, shots // groups)]
     for i, g in enumerate(whole):
         assert rel_l2(g, sum(q[i] for q in parts)) < 2e-5
